@@ -152,6 +152,33 @@ def _fused(fmt, parts, rows, k):
     return weights
 
 
+def _w8a8_inputs(case, g):
+    m, n, k = case["m"], case["n"], case["k"]
+    w = _codes(g, n * k, -127, 128, torch.int8).view(n, k)
+    state = dict(kind="w8a8", azp=case["azp"], m=m, n=n, k=k, w=w,
+                 x=_codes(g, m * k, -127, 128, torch.int8).view(m, k),
+                 ws=_uniform(g, n, 0.001, 0.01), xs=_uniform(g, m, 0.005, 0.05))
+    if case["azp"]:
+        state["row_sum"] = w.sum(dim=1, dtype=torch.int32)
+        state["zp"] = _codes(g, m, -20, 21, torch.int32)
+    return state
+
+
+def _canonical_inputs(case, g):
+    m, n, k = case["m"], case["n"], case["k"]
+    groups = k // case["group"] if case["group"] else 1
+    level = 73.3 if case["layout"] == "int8" else 4.6
+    scales = _uniform(g, n * groups, 0.5, 1.5) / (level * k ** 0.5)
+    if case["layout"] == "int8":
+        data = _codes(g, n * k, -127, 128, torch.int8).view(torch.uint8)
+    else:
+        data = torch.randint(0, 256, (n * k // 2,), generator=g, device="cuda", dtype=torch.uint8)
+    zeros = _codes(g, n * groups, 5, 11, torch.float32) if case["layout"] == "uint4" else None
+    x = torch.randn((m, k), generator=g, device="cuda").to(TYPES[case["x_type"]][1])
+    bias = torch.randn(n, generator=g, device="cuda") * 0.1 if case["bias"] else None
+    return data, scales, zeros, x, bias
+
+
 def prepare(case, seed):
     g = _generator(seed)
     kind = case["kind"]
@@ -180,36 +207,20 @@ def prepare(case, seed):
             x = x.bfloat16().view(torch.int16)
         return dict(kind=kind, weights=weights, m=m, x=x, y=torch.zeros((m, n), device="cuda"))
     if kind == "w8a8":
-        w = _codes(g, n * k, -127, 128, torch.int8).view(n, k)
-        state = dict(kind=kind, azp=case["azp"], m=m, n=n, k=k, w=w,
-                     x=_codes(g, m * k, -127, 128, torch.int8).view(m, k),
-                     ws=_uniform(g, n, 0.001, 0.01), xs=_uniform(g, m, 0.005, 0.05),
-                     y=torch.zeros((m, n), device="cuda"))
-        if case["azp"]:
-            state["row_sum"] = w.sum(dim=1, dtype=torch.int32)
-            state["zp"] = _codes(g, m, -20, 21, torch.int32)
-        return state
+        return dict(_w8a8_inputs(case, g), y=torch.zeros((m, n), device="cuda"))
     if kind == "canonical":
         layout = {"int8": qx.INT8_SYMMETRIC, "uint4": qx.UINT4_AFFINE, "int4": qx.INT4_SYMMETRIC}[case["layout"]]
-        groups = k // case["group"] if case["group"] else 1
-        level = 73.3 if case["layout"] == "int8" else 4.6
-        scales = _uniform(g, n * groups, 0.5, 1.5) / (level * k ** 0.5)
-        if case["layout"] == "int8":
-            data = _codes(g, n * k, -127, 128, torch.int8).view(torch.uint8)
-        else:
-            data = torch.randint(0, 256, (n * k // 2,), generator=g, device="cuda", dtype=torch.uint8)
-        zeros = _codes(g, n * groups, 5, 11, torch.float32).cpu().numpy() if case["layout"] == "uint4" else None
+        data, scales, zeros, x, bias = _canonical_inputs(case, g)
         host = (data.cpu().numpy(), scales.cpu().numpy())
         mode = qx.SCALE_GROUP if case["group"] else qx.SCALE_CHANNEL
         weights = qx.CanonicalWeights()
-        qx.check(weights.prepare(qx.canonical_view(layout, mode, n, k, case["group"] or k, *host, zeros=zeros)),
+        qx.check(weights.prepare(qx.canonical_view(layout, mode, n, k, case["group"] or k, *host,
+                                                    zeros=None if zeros is None else zeros.cpu().numpy())),
                  "prepare")
-        x_type, x_torch = TYPES[case["x_type"]]
+        x_type = TYPES[case["x_type"]][0]
         y_type, y_torch = TYPES[case["y_type"]]
         return dict(kind=kind, weights=weights, m=m, x_type=x_type, y_type=y_type,
-                    x=torch.randn((m, k), generator=g, device="cuda").to(x_torch),
-                    y=torch.zeros((m, n), device="cuda", dtype=y_torch),
-                    bias=torch.randn(n, generator=g, device="cuda") * 0.1 if case["bias"] else None,
+                    x=x, y=torch.zeros((m, n), device="cuda", dtype=y_torch), bias=bias,
                     activation=ACTIVATIONS[case["activation"]])
     packed = torch.randint(0, 256, (n * k // 2,), generator=g, device="cuda", dtype=torch.uint8)
     return dict(kind=kind, m=m, n=n, k=k, packed=packed,
@@ -295,3 +306,79 @@ def tolerance(case):
     if kind == "canonical" and case["y_type"] != "f32":
         return {"rel": 5e-4, "max": 1e-2} if case["y_type"] == "bf16" else {"rel": 6e-5, "max": 1.3e-3}
     return {"rel": 4e-6, "max": 4e-5}  # 32-bit sums
+
+
+# ---- the same values in 64 bits ---------------------------------------------------------------
+
+def _dense_blocks(fmt, blocks, n, k):
+    b = blocks.view(n, k // 32, -1)
+    d = b[..., :2].contiguous().view(torch.float16).double()
+    if fmt == Q8_0:
+        codes = b[..., 2:].contiguous().view(torch.int8).double()
+    else:
+        codes = torch.cat((b[..., 2:] & 15, b[..., 2:] >> 4), dim=-1).double() - 8.0
+    return (d * codes).view(n, k)
+
+
+def _dense_nibbles(packed, n, k):
+    b = packed.view(n, k // 2)
+    return torch.stack((b & 15, b >> 4), dim=-1).view(n, k).double()
+
+
+def _activate(v, activation):
+    if activation == "gelu_erf":
+        return torch.nn.functional.gelu(v)
+    if activation == "gelu_tanh":
+        return torch.nn.functional.gelu(v, approximate="tanh")
+    if activation == "silu":
+        return torch.nn.functional.silu(v)
+    return torch.relu(v) ** 2 if activation == "relu2" else v
+
+
+def exact(case, seed):
+    g = _generator(seed)
+    kind = case["kind"]
+    if kind == "layer":  # the draws of prepare(), in its order
+        fmt, h, kv, ffn = FORMATS[case["fmt"]], case["hidden"], case["kv"], case["ffn"]
+        over_h, over_f = _layer_scale(fmt, h), _layer_scale(fmt, ffn)
+        wq, wk, wv = (_dense_blocks(fmt, _blocks(g, fmt, n, h, *over_h), n, h) for n in (h, kv, kv))
+        up, gate = (_dense_blocks(fmt, _blocks(g, fmt, ffn, h, *over_h), ffn, h) for _ in range(2))
+        wo = _dense_blocks(fmt, _blocks(g, fmt, h, h, *over_h), h, h)
+        down = _dense_blocks(fmt, _blocks(g, fmt, h, ffn, *over_f), h, ffn)
+        x = torch.randn((1, h), generator=g, device="cuda").double()
+        q, key, value = x @ wq.T, x @ wk.T, x @ wv.T
+        a = q @ wo.T
+        mid = torch.nn.functional.silu(a @ gate.T) * (a @ up.T)
+        return q, key, value, mid[0], mid @ down.T
+    m, n, k = case["m"], case["n"], case["k"]
+    if kind in ("gemm", "host", "prefill"):
+        fmt = FORMATS[case["fmt"]]
+        w = _dense_blocks(fmt, _blocks(g, fmt, n, k, *SCALES[fmt]), n, k)
+        x = torch.randn((m, k), generator=g, device="cuda")
+        y = (x.bfloat16() if kind == "prefill" else x).double() @ w.T
+        return y.cpu().numpy() if kind == "host" else y
+    if kind == "w8a8":
+        s = _w8a8_inputs(case, g)
+        acc = s["x"].double() @ s["w"].double().T
+        if case["azp"]:
+            acc -= s["zp"].double()[:, None] * s["row_sum"].double()[None, :]
+        return acc * s["ws"].double()[None, :] * s["xs"].double()[:, None]
+    if kind == "canonical":
+        data, scales, zeros, x, bias = _canonical_inputs(case, g)
+        w = data.view(torch.int8).view(n, k).double() if case["layout"] == "int8" else _dense_nibbles(data, n, k)
+        if case["layout"] == "int4":
+            w = torch.where(w >= 8, w - 16, w)
+        w = w.view(n, scales.numel() // n, -1)
+        if zeros is not None:
+            w = w - zeros.double().view(n, -1, 1)
+        w = (w * scales.double().view(n, -1, 1)).view(n, k)
+        y = x.double() @ w.T
+        return _activate(y if bias is None else y + bias.double(), case["activation"])
+    packed = torch.randint(0, 256, (n * k // 2,), generator=g, device="cuda", dtype=torch.uint8)
+    ws = _uniform(g, n, 0.5, 1.5) / (4.6 * k ** 0.5)
+    x = torch.randn((m, k), generator=g, device="cuda")
+    # the int8 activation codes are part of the operation: one scale per token, rounded in 32 bits
+    xs = x.abs().amax(dim=1, keepdim=True) / 127.0
+    codes = torch.round(x * (1.0 / xs)).clamp(-127, 127)
+    acc = codes.double() @ (_dense_nibbles(packed, n, k) - 8.0).T
+    return acc * ws.double()[None, :] * xs.double()
