@@ -211,11 +211,12 @@ def prepare(case, seed):
     if kind == "canonical":
         layout = {"int8": qx.INT8_SYMMETRIC, "uint4": qx.UINT4_AFFINE, "int4": qx.INT4_SYMMETRIC}[case["layout"]]
         data, scales, zeros, x, bias = _canonical_inputs(case, g)
+        # (host arrays of its own: a view points into them)
         host = (data.cpu().numpy(), scales.cpu().numpy())
+        zeros = None if zeros is None else zeros.cpu().numpy()
         mode = qx.SCALE_GROUP if case["group"] else qx.SCALE_CHANNEL
         weights = qx.CanonicalWeights()
-        qx.check(weights.prepare(qx.canonical_view(layout, mode, n, k, case["group"] or k, *host,
-                                                    zeros=None if zeros is None else zeros.cpu().numpy())),
+        qx.check(weights.prepare(qx.canonical_view(layout, mode, n, k, case["group"] or k, *host, zeros=zeros)),
                  "prepare")
         x_type = TYPES[case["x_type"]][0]
         y_type, y_torch = TYPES[case["y_type"]]
