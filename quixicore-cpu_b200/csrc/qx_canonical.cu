@@ -56,6 +56,7 @@
 #include "qx_common.cuh"
 #include "qx_gemv.cuh"
 #include "qx_int8_gemm.cuh"
+#include "qx_scaled_gemm.cuh"
 
 struct qx_canonical_weights {
   int layout = 0;
@@ -101,39 +102,13 @@ __device__ __forceinline__ float load_storage(const void* base, int type, long l
   return __uint_as_float(static_cast<uint32_t>(bits) << 16);
 }
 
-// float_to_bf16 of the reference (kernels/utils/float_storage_ref.cpp:184-193): round to
-// nearest even on the bit pattern; a NaN keeps its upper payload with the quiet bit set.
-__device__ __forceinline__ uint16_t to_bf16_bits(float value) {
-  const uint32_t bits = __float_as_uint(value);
-  if ((bits & 0x7f800000u) == 0x7f800000u && (bits & 0x007fffffu) != 0) {
-    return static_cast<uint16_t>((bits >> 16) | 0x0040u);
-  }
-  return static_cast<uint16_t>((bits + 0x7fffu + ((bits >> 16) & 1u)) >> 16);
-}
-
 __device__ __forceinline__ void store_storage(void* base, int type, long long index, float value) {
   if (type == QX_STORAGE_F32) {
     static_cast<float*>(base)[index] = value;
   } else if (type == QX_STORAGE_F16) {
     static_cast<uint16_t*>(base)[index] = __half_as_ushort(__float2half_rn(value));
   } else {
-    static_cast<uint16_t*>(base)[index] = to_bf16_bits(value);
-  }
-}
-
-// projection_activation, qgemm_canonical.cpp:361-379
-__device__ __forceinline__ float apply_activation(float v, int activation) {
-  switch (activation) {
-    case QX_ACTIVATION_GELU_ERF:
-      return 0.5f * v * (1.0f + erff(v * 0.7071067811865475f));
-    case QX_ACTIVATION_GELU_TANH:
-      return 0.5f * v * (1.0f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));
-    case QX_ACTIVATION_SILU:
-      return v / (1.0f + expf(-v));
-    case QX_ACTIVATION_RELU2:
-      return v > 0.0f ? v * v : 0.0f;
-    default:
-      return v;
+    static_cast<uint16_t*>(base)[index] = storage_bf16_bits(value);
   }
 }
 
@@ -371,7 +346,7 @@ __global__ void __launch_bounds__(32 * WARPS) canonical_gemm_kernel(const Canoni
       const long long row = row0 + r;
       if (lane == ((r * TM + t) & 31) && row_ok[r] && t < tokens) {
         if (p.bias != nullptr) v += p.bias[row];
-        v = apply_activation(v, p.activation);
+        v = projection_activation(v, p.activation);
         store_storage(p.y, p.y_type, (token0 + t) * p.rows + row, v);
       }
     }
@@ -724,7 +699,7 @@ __global__ void __launch_bounds__(32 * kDigitWarps) canonical_digits_kernel(
       const long long row = row0 + r;
       if (lane == ((r * TM + t) & 31) && row_ok[r] && t < tokens) {
         if (p.bias != nullptr) v += p.bias[row];
-        v = apply_activation(v, p.activation);
+        v = projection_activation(v, p.activation);
         store_storage(p.y, p.y_type, (token0 + t) * p.rows + row, v);
       }
     }
@@ -944,7 +919,7 @@ __global__ void __launch_bounds__(256) canonical_combine_kernel(
     for (int d = kPlanes - 2; d >= 0; --d) v += partial[d * plane + i];
     const long long token = i / rows, row = i - token * rows;
     if (bias != nullptr) v += bias[row];
-    store_storage(y, y_type, token * ldy + row, apply_activation(v, activation));
+    store_storage(y, y_type, token * ldy + row, projection_activation(v, activation));
   }
 }
 
@@ -1020,6 +995,26 @@ qx_status launch_any(const CanonicalParams& p, bool digits, uint32_t* image, int
   return launch_layout<LAYOUT>(p, sm_count, stream);
 }
 
+// Which batches take the tensor cores with scales applied per group (qx_scaled_gemm.cu).
+// Measured there | here (us, bf16 tokens unless noted):
+//   uint4, groups of 128, 14336 x 4096:  4 tokens 32.9 | 36.7,  5: 33.5 | 61.7,  512: 129 | 3592
+//   4096 x 4096:  4 tokens 18.2 | 16.9,  5: 19.3 | 26.8,  128: 30 | 272
+//   f32 activations (three planes), groups of 32, 14336 x 4096: 25 tokens 66.7 | 200;
+//   1024 x 1024: 32 tokens 15.7 | 13.3,  64: 17.9 | 19.2
+//   int8 with one scale per row against the digit planes below, 14336 x 4096: 64 tokens
+//   33.0 | 31.1,  128: 39.0 | 47.6,  512: 109 | 169;  4096 x 4096: 128 tokens 28.4 | 27.7
+bool scaled_route(const qx_canonical_weights* w, int x_type, long long m) {
+  // a tile is 128 weight rows: smaller matrices would be mostly padding
+  if (w->group_index != nullptr || w->rows < 128) return false;
+  // fractional zero points have no exact 16-bit form
+  if (w->layout == QX_CANONICAL_UINT4_AFFINE && !w->integral_zeros) return false;
+  const long long work = m * w->rows * w->columns;
+  if (w->layout == QX_CANONICAL_INT8_SYMMETRIC && w->groups_per_row == 1) {
+    return x_type != QX_STORAGE_F32 && work >= (1LL << 32);
+  }
+  return x_type == QX_STORAGE_F32 ? m >= 25 && work >= (1LL << 26) : m >= 5 && work >= (1LL << 25);
+}
+
 qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_type,
                            const float* bias, void* y, int y_type, long long m, int activation,
                            qx_workspace* workspace, cudaStream_t stream) {
@@ -1061,6 +1056,31 @@ qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_t
   // float multiply-adds on weights decoded one by one
   const bool digits = w->group_index == nullptr &&
                       (p.groups_per_row == 1 || p.group_size % kElems == 0);
+  // batches on the tensor cores with the scales applied per group (qx_scaled_gemm.cu)
+  ScaledGemmArgs scaled{};
+  scaled.source = int8 ? kScaledBytes : kScaledNibbles;
+  scaled.codes = w->data;
+  scaled.scales = w->scales;
+  scaled.zeros = w->zeros;
+  scaled.nibble_xor = w->layout == QX_CANONICAL_INT4_SYMMETRIC ? 0x88888888u : 0u;
+  scaled.rows = w->rows;
+  scaled.columns = w->columns;
+  scaled.group = p.groups_per_row == 1 ? w->columns : w->group_size;
+  scaled.x = x;
+  scaled.x_type = x_type;
+  scaled.order = w->act_order;
+  scaled.m = m;
+  scaled.bias = bias;
+  scaled.activation = activation;
+  scaled.y = y;
+  scaled.y_type = y_type;
+  scaled.ldy = w->rows;
+  if (scaled_route(w, x_type, m) && scaled_gemm_serves(scaled)) {
+    const int sm_count = ctx->prop.multiProcessorCount;
+    QX_TRY(workspace->reserve(kWorkspaceCounterBytes + scaled_gemm_scratch_bytes(scaled, sm_count)));
+    return launch_scaled_gemm(scaled, static_cast<uint8_t*>(workspace->base) + kWorkspaceCounterBytes,
+                              static_cast<int*>(workspace->base), sm_count, ctx->error_dev, stream);
+  }
   // workspace behind its counters: [gathered activations (act-order)][digit images]
   const size_t gather_bytes =
       w->act_order != nullptr ? align_up(static_cast<size_t>(m) * w->columns * sizeof(float), 256) : 0;

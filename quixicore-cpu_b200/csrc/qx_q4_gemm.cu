@@ -23,14 +23,15 @@
 // Rounding: the weight d * (nibble - 8) is one fp16 multiply of the block's own fp16 scale
 // (relative error at most 2^-12 per weight); products are exact and sums f32 in the tensor
 // core. This is the stated 1e-2 tolerance class of the 4-bit prefill path (measured: about
-// 2e-4 of a row's rms); batches below 64 rows and q8_0 weights take the exact digit
-// kernels instead.
+// 2e-4 of a row's rms); batches below 64 rows take the exact digit kernels instead, and q8_0
+// weights those or, from 16 rows on, the scaled-projection kernel (qx_scaled_gemm.cu).
 
 #include <cuda.h>
 #include <cuda_fp16.h>
 
 #include "qx_gemv.cuh"
 #include "qx_gemv_tc.cuh"
+#include "qx_scaled_gemm.cuh"
 #include "qx_sm100.cuh"
 #include "qx_weights.cuh"
 
@@ -356,6 +357,11 @@ q4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const Q4GemmParams 
   }
 }
 
+// q8_0 panels take the scaled-projection kernel (qx_scaled_gemm.cu) from this many tokens on:
+// 14336 x 4096, 16 tokens 37.5 us against 39.0 on the digit kernels, 24: 37.9 against 62.1;
+// 4096 x 11008, 16 tokens 34.1 against 35.9, 331: 102 against 667.
+constexpr long long kScaledPrefillRows = 16;
+
 constexpr size_t kQ4GemmSmem = 1024 + kASlots * kABytes + kBSlots * kMaxTokens * 128 +
                                kRawSlots * kRawBytes + sizeof(Q4GemmBarriers) + 64;
 
@@ -454,6 +460,29 @@ qx_status launch_q4_gemm_bf16(const qx_weights* w, const uint16_t* x_bf16_dev, f
   if (w->format == QX_FORMAT_Q4_0 && m >= 64 && w->tiles < (1LL << 20) && m < (1LL << 30) &&
       m * w->columns < (1LL << 40)) {
     return launch_tc(w, x_bf16_dev, y_dev, m, ldy, ws, stream);
+  }
+  if (w->format == QX_FORMAT_Q8_0 && w->segments == 1 && m >= kScaledPrefillRows) {
+    ScaledGemmArgs a{};
+    a.source = kScaledPanelQ8;
+    a.codes = w->panel;
+    a.rows = w->rows;
+    a.columns = w->columns;
+    a.group = 32;
+    a.x = x_bf16_dev;
+    a.x_type = QX_STORAGE_BF16;
+    a.m = m;
+    a.activation = QX_ACTIVATION_NONE;
+    a.y = y_dev;
+    a.y_type = QX_STORAGE_F32;
+    a.ldy = ldy;
+    if (scaled_gemm_serves(a)) {
+      DeviceContext* ctx = nullptr;
+      QX_TRY(current_context(&ctx));
+      const int sm_count = ctx->prop.multiProcessorCount;
+      QX_TRY(ws->reserve(kWorkspaceCounterBytes + scaled_gemm_scratch_bytes(a, sm_count)));
+      return launch_scaled_gemm(a, static_cast<uint8_t*>(ws->base) + kWorkspaceCounterBytes,
+                                static_cast<int*>(ws->base), sm_count, ctx->error_dev, stream);
+    }
   }
   // Exact path: widen the activations to f32 (bf16 -> f32 is exact) and reuse the f32
   // batched kernel; its scratch sits at the start of the workspace and the widened copy

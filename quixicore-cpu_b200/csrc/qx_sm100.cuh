@@ -78,6 +78,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   }
 }
 
+// The same by a whole warp, with one outcome for all its lanes (they go on to warp-wide loads).
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+
 // Records why a kernel gives up (role / barrier code) in the caller's error word, which may
 // be host memory mapped into the device's address space: plain accesses only, first code
 // wins (approximately: concurrent reporters may overwrite each other, any of them will do).

@@ -1,0 +1,98 @@
+// Pieces shared by the persistent tensor-core kernels whose weights are converted to 16-bit
+// operands on the way (qx_scaled_gemm.cu, qx_gemv_batch.cu): ring positions, bulk copies,
+// packed f32 arithmetic and the exact conversions of integer codes.
+#pragma once
+
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include "qx_sm100.cuh"
+
+namespace qx {
+namespace tile {
+
+struct Ring {
+  uint32_t slot = 0, phase = 0;
+  __device__ __forceinline__ void advance(uint32_t slots) {
+    if (++slot == slots) {
+      slot = 0;
+      phase ^= 1u;
+    }
+  }
+};
+
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+      ::"r"(sm100::smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(sm100::smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void wait_for_kernel_in_front() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// ---- two f32 values in a 64-bit register -------------------------------------------------
+__device__ __forceinline__ unsigned long long pack2(uint32_t lo, uint32_t hi) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+  return v;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
+  uint32_t a, b;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(v));
+  lo = __uint_as_float(a);
+  hi = __uint_as_float(b);
+}
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long v;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
+
+// ---- 16-bit whole numbers ----------------------------------------------------------------
+__device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
+  const __half2 v = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+template <bool BF16>
+__device__ __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) {
+  if (BF16) {
+    const __nv_bfloat162 v = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&a),
+                                     *reinterpret_cast<const __nv_bfloat162*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&v);
+  }
+  const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+// Two signed bytes of `w` picked by `selector` -> two 16-bit whole numbers.
+template <bool BF16>
+__device__ __forceinline__ uint32_t convert_bytes2(uint32_t w, uint32_t selector) {
+  if (BF16) {
+    // (128 + low seven bits) - (128, or 256 for a negative code)
+    const uint32_t p = __byte_perm(w, 0x43434343u, selector);
+    return sub2<true>(p & 0xFF7FFF7Fu, p & 0xFF80FF80u);
+  }
+  // code ^ 0x80 = code + 128 under the exponent of 1024
+  const uint32_t p = __byte_perm(w ^ 0x80808080u, 0x64646464u, selector);
+  return sub2<false>(p, 0x64806480u);
+}
+
+// ---- TMEM: 32 lanes x 16 consecutive columns ----------------------------------------
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { sm100::tmem_ld_32x16(taddr, r); }
+
+// 16 columns into the first half of `r`
+__device__ __forceinline__ void tmem_ld_32x16_low(uint32_t taddr, uint32_t (&r)[32]) {
+  uint32_t low[16];
+  sm100::tmem_ld_32x16(taddr, low);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    r[i] = low[i];
+    r[16 + i] = 0u;
+  }
+}
+
+}  // namespace tile
+}  // namespace qx

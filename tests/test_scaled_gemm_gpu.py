@@ -1,0 +1,123 @@
+"""Batched projections on the tensor cores with scales along K (csrc/qx_scaled_gemm.cu), through
+the C ABI: canonical int4 / uint4 / int8 tensors and q8_0 panels with 16-bit activations.
+
+Every product is exact and every group is scaled in f32, so the tolerance is that of f32 sums, the
+rule of the reference's own projection test: 4e-5 * (1 + |exact|) against float64.
+"""
+
+import numpy as np
+import pytest
+
+from test_canonical_gpu import BF16, F16, F32, INT4, INT8, OUT_TOLERANCE, UINT4, activation_f64, close, widen
+
+pytestmark = pytest.mark.gpu
+
+GROUP, CHANNEL = 4, 3
+
+
+def _storage(x, x_type):
+    """(activations as the entry point takes them, the same values as f32)"""
+    import torch
+    if x_type == F32:
+        return x, x
+    t = torch.from_numpy(x).to(torch.float16 if x_type == F16 else torch.bfloat16)
+    return np.ascontiguousarray(t.view(torch.int16).numpy().view(np.uint16)), t.float().numpy()
+
+
+def _tensor(qx, oracle_mod, rng, layout, group, n, k, act_order=None):
+    groups = k // group if group else 1
+    mode = GROUP if group else CHANNEL
+    codes = n * k if layout == INT8 else n * k // 2
+    data = rng.integers(0, 256, codes, dtype=np.uint8)
+    scales = rng.uniform(0.002, 0.03, n * groups).astype(np.float32)
+    zeros = rng.integers(0, 16, n * groups).astype(np.float32) if layout == UINT4 else None
+    view = qx.canonical_view(layout, mode, n, k, group or k, data, scales, zeros=zeros, act_order=act_order)
+    weights = qx.CanonicalWeights()
+    assert weights.prepare(view) == qx.OK, qx.last_error()
+    return weights, oracle_mod.CanonicalTensor(layout, mode, n, k, group or k, data, scales, zeros, None, act_order)
+
+
+@pytest.mark.parametrize("layout,group,n,k,m,x_type", [
+    (UINT4, 128, 4097, 2048, 5, BF16),   # smallest batch, a last tile of one row
+    (UINT4, 128, 1025, 1152, 32, F16),   # half a slab at the end
+    (INT4, 32, 1000, 1056, 33, BF16),    # 33 groups: the last stage holds groups of padding
+    (UINT4, 32, 1100, 992, 64, F32),     # three planes, largest small tile
+    (INT4, 64, 260, 2112, 65, F16),      # first large tile
+    (UINT4, 96, 256, 1152, 130, BF16),   # groups that do not divide a slab
+    (INT4, 0, 384, 800, 257, F32),       # one scale per row, tokens in five tiles
+    (UINT4, 256, 640, 2560, 300, BF16),  # groups larger than an accumulator's columns
+    (INT8, 64, 900, 1088, 70, F32),      # bytes: half a slot at the end
+    (INT8, 0, 4100, 2064, 512, BF16),    # bytes with one scale per row: rows of 129 vectors
+])
+def test_batches_against_float64(qx, orc, oracle_mod, layout, group, n, k, m, x_type):
+    rng = np.random.Generator(np.random.Philox(key=[n * 31 + k, m * 7 + group]))
+    weights, tensor = _tensor(qx, oracle_mod, rng, layout, group, n, k)
+    x, x_exact = _storage((rng.standard_normal((m, k)) * 0.1).astype(np.float32), x_type)
+    bias = rng.standard_normal(n).astype(np.float32)
+    exact = orc.canonical_gemm_f64(tensor, np.ascontiguousarray(x_exact), F32, m)
+    status, y = weights.qgemm_storage(x, x_type, m)
+    assert status == qx.OK, qx.last_error()
+    assert close(y, exact)
+    status, typed = weights.qgemm_storage(x, x_type, m, y_type=BF16, bias=bias, activation=3)
+    assert status == qx.OK, qx.last_error()
+    assert close(widen(typed, BF16), activation_f64(exact + bias.astype(np.float64)[None, :], 3), OUT_TOLERANCE[BF16])
+    status, again = weights.qgemm_storage(x, x_type, m)  # pieces of a tile are added in a fixed order
+    assert status == qx.OK and np.array_equal(again.view(np.uint32), y.view(np.uint32))
+    assert qx.lib.qx_check_device_errors() == qx.OK, qx.last_error()
+
+
+def test_act_order_and_unaligned_activations(qx, orc, oracle_mod):
+    import torch
+    n, k, m = 900, 1024, 40
+    rng = np.random.Generator(np.random.Philox(key=[5, 6]))
+    order = rng.permutation(k).astype(np.int32)
+    weights, tensor = _tensor(qx, oracle_mod, rng, INT4, 128, n, k, act_order=order)
+    plain, plain_tensor = _tensor(qx, oracle_mod, rng, INT4, 128, n, k)
+    x, x_exact = _storage((rng.standard_normal((m, k)) * 0.1).astype(np.float32), BF16)
+    status, y = weights.qgemm_storage(x, BF16, m)
+    assert status == qx.OK, qx.last_error()
+    assert close(y, orc.canonical_gemm_f64(tensor, np.ascontiguousarray(x_exact), F32, m))
+    # device activations that start two bytes past a 16-byte boundary
+    buffer = torch.zeros(m * k + 8, dtype=torch.int16, device="cuda")
+    shifted = buffer[1:1 + m * k].view(m, k)
+    shifted.copy_(torch.from_numpy(x.view(np.int16)))
+    out = torch.zeros((m, n), device="cuda")
+    assert plain.qgemm_storage_dev(shifted, BF16, out, F32, m) == qx.OK, qx.last_error()
+    torch.cuda.synchronize()
+    assert close(out.cpu().numpy(), orc.canonical_gemm_f64(plain_tensor, np.ascontiguousarray(x_exact), F32, m))
+
+
+def test_a_token_that_is_not_finite_stays_alone(qx, orc, oracle_mod):
+    n, k, m = 2048, 1024, 33
+    rng = np.random.Generator(np.random.Philox(key=[8, 9]))
+    weights, tensor = _tensor(qx, oracle_mod, rng, UINT4, 64, n, k)
+    x = (rng.standard_normal((m, k)) * 0.1).astype(np.float32)
+    x[4, 17] = np.nan
+    for x_type in (F32, BF16):
+        stored, values = _storage(x, x_type)
+        status, y = weights.qgemm_storage(stored, x_type, m)
+        assert status == qx.OK, qx.last_error()
+        assert np.all(np.isnan(y[4]))
+        finite = [r for r in range(m) if r != 4]
+        exact = orc.canonical_gemm_f64(tensor, np.ascontiguousarray(values[finite]), F32, m - 1)
+        assert close(y[finite], exact)
+
+
+@pytest.mark.parametrize("n,k,m", [(128, 256, 16), (300, 1056, 33), (257, 416, 64), (640, 2080, 65), (384, 11008, 331)])
+def test_q8_0_prefill(qx, orc, wl, n, k, m):
+    import torch
+    packed = wl.packed_blocks(0, n, k, 0.001, 0.02, seed=n + k)
+    xb = wl.to_bf16_bits(wl.activations_f32(m, k, seed=m))
+    weights = qx.PackedWeights()
+    assert weights.prepare(0, packed, n, k) == qx.OK, qx.last_error()
+    y = torch.full((m, n + 3), -7.0, device="cuda")  # a row stride of its own
+    status = weights.qgemm_bf16_dev(torch.from_numpy(xb.view(np.int16)).cuda(), y, m, ldy=n + 3)
+    assert status == qx.OK, qx.last_error()
+    torch.cuda.synchronize()
+    got = y.cpu().numpy()
+    assert np.all(got[:, n:] == -7.0)
+    _, exact = orc.qgemm_f64(0, packed, wl.bf16_bits_to_f32(xb), m, n, k)
+    # K terms of f32 sums: at most K / 32 roundings of 2^-24 of the running sum, which stays below
+    # the sum of the magnitudes; 4e-6 of a row's rms is four times what is measured
+    rms = np.sqrt((exact ** 2).mean(axis=1, keepdims=True))
+    assert np.all(np.abs(got[:, :n] - exact) <= 4e-6 * (np.abs(exact) + rms))
