@@ -1,0 +1,36 @@
+"""W4A8 on the tensor cores (csrc/qx_scaled_gemm.cu from qx_lowbit_gemm_w8a8): f16 whole numbers with
+sums below 2^24, so the result keeps every bit of the reference's
+(tests/correctness/test_lowbit_w8a8.cpp:53-72 demands exact equality)."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (2, 128, 258),      # smallest batch and matrix of rows that start on any byte
+    (13, 128, 256),     # ... and of rows on whole vectors
+    (1, 4096, 2050),    # one row of a large matrix
+    (33, 129, 1033),    # an odd number of columns; a second tile of one row
+    (64, 300, 2050),
+    (65, 257, 1502),    # first large tile
+    (130, 200, 1312),   # whole tiles only
+    (5, 128, 16510),    # sums up to the largest that stay below 2^24
+    (5, 128, 16514),    # one step further: the integer kernel
+])
+def test_bits_of_the_reference(qx, orc, m, n, k):
+    rng = np.random.Generator(np.random.Philox(key=[m * 1000 + n, k]))
+    packed = rng.integers(0, 256, (n, (k + 1) // 2), dtype=np.uint8)
+    if k >= 16000:  # the largest sums: every product is -8 * 127 or 8 * 127
+        packed[:] = 0
+    scales = rng.uniform(0.001, 0.1, n).astype(np.float32)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    if k >= 16000:
+        x = np.ones_like(x)
+    x[m // 2, ::5] = 0.0
+    status, y = qx.lowbit_gemm_w8a8(packed.reshape(-1), scales, x, m, n, k)
+    assert status == qx.OK, qx.last_error()
+    _, want = orc.lowbit_gemm_w8a8(packed.reshape(-1), scales, x, m, n, k)
+    assert np.array_equal(np.asarray(y).view(np.uint32).reshape(m, n), np.asarray(want).view(np.uint32).reshape(m, n))
+    assert qx.lib.qx_check_device_errors() == qx.OK, qx.last_error()
