@@ -27,6 +27,8 @@
 // With an act-order map the activations are first gathered into packed column order.
 //   tensor cores (int8 with one scale per row, five tokens or more): four digit planes under a
 //           per-token envelope through the W8A8 GEMM; see "long prefills" below.
+//   tensor cores with scales applied per group (batches of the 4-bit and group-scaled tensors,
+//           long prompts of row-scaled int8): qx_scaled_gemm.cu, chosen by scaled_route below.
 // Inputs stored as f16 / bf16 are widened exactly, the output is rounded once at the store.
 // On the first two paths a token's result does not depend on the batch it is computed in; a
 // batch that crosses five tokens changes route and with it the rounding (same tolerance).

@@ -11,7 +11,8 @@
 //
 // Both matmuls are weight-streaming kernels for decode-sized batches: a warp owns an output
 // channel, lanes read 16 bytes (32 weights) at a time, the weights are read ONCE for up to
-// MT activation rows. W4A8 multiplies with dp4a (the nibbles of a word as two unsigned
+// MT activation rows; W4A8 batches go to the tensor cores instead (see "W4A8 on the tensor
+// cores"). W4A8 multiplies with dp4a (the nibbles of a word as two unsigned
 // operands against the even / odd activation codes, the -8 folded into 8 * sum(codes) per
 // row) and reproduces the reference bit for bit: exact int32 dot, then
 // float(dot) * weight_scale * activation_scale as two rounded multiplies.

@@ -1,6 +1,6 @@
-// Pieces shared by the persistent tensor-core kernels whose weights are converted to 16-bit
-// operands on the way (qx_scaled_gemm.cu, qx_gemv_batch.cu): ring positions, bulk copies,
-// packed f32 arithmetic and the exact conversions of integer codes.
+// Pieces of the persistent tensor-core kernel whose weights are converted to 16-bit operands on
+// the way (qx_scaled_gemm.cu): ring positions, bulk copies, packed f32 arithmetic and the exact
+// conversions of integer codes.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -46,17 +46,8 @@ __device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& 
 __device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-  unsigned long long v;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
-  return v;
-}
 
 // ---- 16-bit whole numbers ----------------------------------------------------------------
-__device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
-  const __half2 v = __floats2half2_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
 template <bool BF16>
 __device__ __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) {
   if (BF16) {
@@ -80,9 +71,7 @@ __device__ __forceinline__ uint32_t convert_bytes2(uint32_t w, uint32_t selector
   return sub2<false>(p, 0x64806480u);
 }
 
-// ---- TMEM: 32 lanes x 16 consecutive columns ----------------------------------------
-__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { sm100::tmem_ld_32x16(taddr, r); }
-
+// ---- TMEM -------------------------------------------------------------------------------
 // 16 columns into the first half of `r`
 __device__ __forceinline__ void tmem_ld_32x16_low(uint32_t taddr, uint32_t (&r)[32]) {
   uint32_t low[16];
