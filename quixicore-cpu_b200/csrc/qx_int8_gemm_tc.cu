@@ -203,6 +203,12 @@ __global__ void __launch_bounds__(kThreads, 1) int8_gemm_tc_kernel(
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = bars->tmem_base;
+  // Launched programmatically: the set-up above may run beside the end of the kernel in front,
+  // nothing is read or written before that one has finished. The kernel behind may start its own
+  // once every CTA of this one holds its tensor memory (after the allocation, so that a CTA of
+  // the next kernel cannot take it first and then wait for this kernel).
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 
   const int total_tiles = p.o_tiles * p.r_tiles;
   const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) |
@@ -485,9 +491,18 @@ qx_status launch_tc_na(const CUtensorMap& map_w, const CUtensorMap& map_x, const
                        int grid, cudaStream_t stream) {
   static SmemOptIn opt_in;
   QX_TRY(opt_in.ensure(int8_gemm_tc_kernel<NA>, tc_smem_bytes(NA, 256)));
-  int8_gemm_tc_kernel<NA><<<grid, kThreads, tc_smem_bytes(NA, p.bn), stream>>>(map_w, map_x, p);
+  cudaLaunchAttribute attribute{};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(static_cast<unsigned>(grid));
+  config.blockDim = dim3(kThreads);
+  config.dynamicSmemBytes = tc_smem_bytes(NA, p.bn);
+  config.stream = stream;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  QX_CUDA_TRY(cudaLaunchKernelEx(&config, int8_gemm_tc_kernel<NA>, map_w, map_x, p));
   count_launch();
-  QX_CUDA_TRY(cudaGetLastError());
   return QX_STATUS_OK;
 }
 
