@@ -999,7 +999,7 @@ qx_status launch_any(const CanonicalParams& p, bool digits, uint32_t* image, int
 
 // Which batches take the tensor cores with scales applied per group (qx_scaled_gemm.cu).
 // Measured there | here (us, bf16 tokens unless noted):
-//   uint4, groups of 128, 14336 x 4096:  4 tokens 32.9 | 36.7,  5: 33.5 | 61.7,  512: 129 | 3592
+//   uint4, groups of 128, 14336 x 4096:  4 tokens 32.9 | 36.7,  5: 33.5 | 61.7,  512: 138 | 3596
 //   4096 x 4096:  4 tokens 18.2 | 16.9,  5: 19.3 | 26.8,  128: 30 | 272
 //   f32 activations (three planes), groups of 32, 14336 x 4096: 25 tokens 66.7 | 200;
 //   1024 x 1024: 32 tokens 15.7 | 13.3,  64: 17.9 | 19.2

@@ -359,7 +359,7 @@ q4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const Q4GemmParams 
 
 // q8_0 panels take the scaled-projection kernel (qx_scaled_gemm.cu) from this many tokens on:
 // 14336 x 4096, 16 tokens 37.5 us against 39.0 on the digit kernels, 24: 37.9 against 62.1;
-// 4096 x 11008, 16 tokens 34.1 against 35.9, 331: 102 against 667.
+// 4096 x 11008, 16 tokens 34.1 against 35.9, 331: 130 against 664.
 constexpr long long kScaledPrefillRows = 16;
 
 constexpr size_t kQ4GemmSmem = 1024 + kASlots * kABytes + kBSlots * kMaxTokens * 128 +
