@@ -1081,7 +1081,8 @@ qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_t
     const int sm_count = ctx->prop.multiProcessorCount;
     QX_TRY(workspace->reserve(kWorkspaceCounterBytes + scaled_gemm_scratch_bytes(scaled, sm_count)));
     return launch_scaled_gemm(scaled, static_cast<uint8_t*>(workspace->base) + kWorkspaceCounterBytes,
-                              static_cast<int*>(workspace->base), sm_count, ctx->error_dev, stream);
+                              static_cast<int*>(workspace->base), kWorkspaceCounterBytes, sm_count,
+                              ctx->error_dev, stream);
   }
   // workspace behind its counters: [gathered activations (act-order)][digit images]
   const size_t gather_bytes =

@@ -486,7 +486,7 @@ qx_status for_row_chunks(long long m, Launch&& launch) {
 // the result is the same two rounded multiplies. Scratch: [f16 codes][scales][counters][pieces].
 constexpr long long kTensorMaxK = 16512;                      // 8 * 127 * k < 2^24
 constexpr int kTensorCtas = 148;                              // pieces of this many CTAs at most
-constexpr size_t kTensorCounterBytes = 2 * kTensorCtas * 8 * sizeof(int);
+constexpr size_t kTensorCounterBytes = scaled_gemm_counter_bytes(kTensorCtas);
 long long code_stride(long long k) { return (k + 7) / 8 * 8; }
 // tiles of more tokens are not cut into pieces (there are enough of them)
 constexpr long long kTensorPieceTokens = 128;
@@ -541,7 +541,7 @@ qx_status launch_w4a8_tensor(const uint8_t* packed, const float* weight_scales, 
   QX_CUDA_TRY(launch_dependent(quantize_codes_f16_kernel, static_cast<unsigned>(m), 256, stream, x, codes, scales,
                                counters, static_cast<int>(kTensorCounterBytes / sizeof(int)), k, code_stride(k)));
   count_launch();
-  return launch_scaled_gemm(a, scratch, counters, ctas, ctx->error_dev, stream);
+  return launch_scaled_gemm(a, scratch, counters, kTensorCounterBytes, ctas, ctx->error_dev, stream);
 }
 
 }  // namespace

@@ -481,7 +481,8 @@ qx_status launch_q4_gemm_bf16(const qx_weights* w, const uint16_t* x_bf16_dev, f
       const int sm_count = ctx->prop.multiProcessorCount;
       QX_TRY(ws->reserve(kWorkspaceCounterBytes + scaled_gemm_scratch_bytes(a, sm_count)));
       return launch_scaled_gemm(a, static_cast<uint8_t*>(ws->base) + kWorkspaceCounterBytes,
-                                static_cast<int*>(ws->base), sm_count, ctx->error_dev, stream);
+                                static_cast<int*>(ws->base), kWorkspaceCounterBytes, sm_count,
+                                ctx->error_dev, stream);
     }
   }
   // Exact path: widen the activations to f32 (bf16 -> f32 is exact) and reuse the f32

@@ -73,7 +73,8 @@ struct Shape {
   static constexpr int kRegShares = R_ISSUE + EPI_ / 4 * R_EPI + CONV_ / 4 * R_CONV;
   static constexpr int kTokens = COLS_ * (EPI_ / 4);  // per tile at most
   static constexpr int kFinishBytes = EPI_ * 32 * kFinishCols * 4;
-  static_assert(RAW_ <= kMaxRaw && CONV_ % 8 == 0 && 65536 / kThreads / 8 * 8 * (kThreads / 128) >= kRegShares, "shape");
+  static_assert(RAW_ <= kMaxRaw && EPI_ <= kScaledEpilogueWarps && CONV_ % 8 == 0 &&
+                    65536 / kThreads / 8 * 8 * (kThreads / 128) >= kRegShares, "shape");
 };
 using Small = Shape<8, 16, 32, 4, 32, 120, 56>;
 using SmallPlanes = Shape<8, 16, 32, 2, 32, 120, 56>;  // three planes: larger stages
@@ -893,9 +894,13 @@ size_t scaled_gemm_scratch_bytes(const ScaledGemmArgs& a, int sm_count) {
   return plan.staged_bytes + plan.partial_bytes;
 }
 
-qx_status launch_scaled_gemm(const ScaledGemmArgs& a, void* scratch, int* counters, int sm_count,
-                             int* error, cudaStream_t stream) {
+qx_status launch_scaled_gemm(const ScaledGemmArgs& a, void* scratch, int* counters, size_t counter_bytes,
+                             int sm_count, int* error, cudaStream_t stream) {
   const Plan plan = make_plan(a, sm_count);
+  if (plan.split && scaled_gemm_counter_bytes(plan.grid) > counter_bytes) {
+    set_last_error_text("scaled projection: more pieces than arrival counters");
+    return QX_STATUS_DEVICE_ERROR;
+  }
   const void* x = a.x;
   if (plan.staged) {
     const long long blocks = (a.m * a.columns + 255) / 256;

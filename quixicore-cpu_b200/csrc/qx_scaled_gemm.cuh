@@ -43,10 +43,16 @@ struct ScaledGemmArgs {
 bool scaled_gemm_serves(const ScaledGemmArgs& a);
 // Scratch behind the workspace's counters that launch_scaled_gemm() uses.
 size_t scaled_gemm_scratch_bytes(const ScaledGemmArgs& a, int sm_count);
-// `scratch`: scaled_gemm_scratch_bytes() bytes, 256-byte aligned; `counters`: the workspace's
-// zeroed counters, left zeroed.
-qx_status launch_scaled_gemm(const ScaledGemmArgs& a, void* scratch, int* counters, int sm_count,
-                             int* error, cudaStream_t stream);
+// Bytes of counters that a launch of at most `ctas` CTAs uses: a CTA holds the first piece of at
+// most two tiles, and every epilogue warp counts for itself.
+constexpr int kScaledEpilogueWarps = 16;  // of the shape that has most of them
+constexpr size_t scaled_gemm_counter_bytes(int ctas) {
+  return 2 * static_cast<size_t>(ctas) * kScaledEpilogueWarps * sizeof(int);
+}
+// `scratch`: scaled_gemm_scratch_bytes() bytes, 256-byte aligned; `counters`: `counter_bytes` of
+// zeroed counters (fewer than the launch needs: QX_STATUS_DEVICE_ERROR), left zeroed.
+qx_status launch_scaled_gemm(const ScaledGemmArgs& a, void* scratch, int* counters, size_t counter_bytes,
+                             int sm_count, int* error, cudaStream_t stream);
 
 // Storage types and activations of a projection's epilogue (qx_canonical.cu), shared.
 __device__ __forceinline__ uint16_t storage_bf16_bits(float value) {

@@ -34,3 +34,44 @@ def test_bits_of_the_reference(qx, orc, m, n, k):
     _, want = orc.lowbit_gemm_w8a8(packed.reshape(-1), scales, x, m, n, k)
     assert np.array_equal(np.asarray(y).view(np.uint32).reshape(m, n), np.asarray(want).view(np.uint32).reshape(m, n))
     assert qx.lib.qx_check_device_errors() == qx.OK, qx.last_error()
+
+
+def _exact(orc, packed, scales, x, m, n, k):
+    """float(dot) * weight scale * activation scale on the oracle's codes; the dots in float64,
+    where they are exact, as the oracle's own loop takes seconds on these sizes."""
+    _, codes, xs = orc.quantize_int8(x, m, k, 0)
+    rows = packed.reshape(n, -1)
+    w = np.stack((rows & 15, rows >> 4), axis=-1).reshape(n, -1)[:, :k].astype(np.float64) - 8.0
+    dot = (codes.reshape(m, k).astype(np.float64) @ w.T).astype(np.float32)
+    return (dot * scales[None, :]) * xs.reshape(m, 1)
+
+
+def _twice_on_one_scratch(qx, packed, scales, x, m, n, k, fill=255):
+    """Two calls of the device entry point on the same scratch, full of `fill` before the first."""
+    import torch
+    scratch = torch.full((int(qx.lib.qx_lowbit_w8a8_scratch_bytes(m, k)),), fill, dtype=torch.uint8, device="cuda")
+    w, ws, xd = (torch.from_numpy(a).cuda() for a in (packed, scales, x))
+    results = []
+    for _ in range(2):
+        y = torch.full((m, n), np.nan, device="cuda")
+        torch.cuda.synchronize()
+        status = qx.lib.qx_lowbit_gemm_w8a8_dev(w.data_ptr(), ws.data_ptr(), xd.data_ptr(), y.data_ptr(),
+                                                scratch.data_ptr(), m, n, k, torch.cuda.current_stream().cuda_stream)
+        assert status == qx.OK, qx.last_error()
+        torch.cuda.synchronize()
+        results.append(y.cpu().numpy())
+    assert qx.lib.qx_check_device_errors() == qx.OK, qx.last_error()
+    return results
+
+
+# tiles cut into pieces on a full grid, so that every CTA's counters are used: 16 epilogue warps
+# from 65 rows on, 8 below
+@pytest.mark.parametrize("m,n,k", [(64, 4096, 4096), (65, 4096, 4096), (100, 4096, 4098), (128, 14336, 4096)])
+def test_pieces_of_a_full_grid(qx, orc, m, n, k):
+    rng = np.random.Generator(np.random.Philox(key=[m, n + k]))
+    packed = rng.integers(0, 256, (n, (k + 1) // 2), dtype=np.uint8)
+    scales = rng.uniform(0.001, 0.1, n).astype(np.float32)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    want = _exact(orc, packed, scales, x, m, n, k)
+    for y in _twice_on_one_scratch(qx, packed, scales, x, m, n, k):
+        assert np.array_equal(y.view(np.uint32), want.view(np.uint32))
