@@ -607,12 +607,16 @@ scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     // -------------------------------- converters --------------------------------
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(S::kConvRegs));
     role = 65;
-    // A thread converts one sub-tile (64 columns) of its row per stage; a group of eight warps
-    // takes every stage, or two groups the first and the second stage of each slab.
+    // A thread converts one sub-tile (64 columns) of its row per stage. A group of eight warps
+    // takes every stage, or two groups take them in turn, strictly, across the ends of tiles as
+    // well: a parity wait is sound only where the phase before it is known to be over. A group
+    // that left out two stages in a row (an odd number of them in a tile, and the next tile's
+    // first one given to the same group again) would take the stage of two rounds ago for free.
     const int cw = warp - 4 - S::kEpi;
     const int r = (cw & 3) * 32 + lane;
     const int sub = (cw >> 2) & 1, group = cw >> 3;
     const int swizzle = r & 7;
+    int turn = 0;  // the group whose stage it is
     Ring raw, st;
     while (ok && walk.next(w)) {
       const int row = w.tile / p.r_tiles * kRows + r;
@@ -627,7 +631,7 @@ scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       bool fetched = false;
       uint32_t base_z = zero_word<BF16>(8.0f);
       if (zeros) {
-        const int column = w.s0 * kSlabK + sub * kSub + (S::kGroups == 2 ? group * kStepCols : 0);
+        const int column = w.s0 * kSlabK + sub * kSub + (S::kGroups == 2 && turn != group ? kStepCols : 0);
         g = column / p.group;
         boundary = (g + 1) * p.group;
         next_zero = g < p.groups ? __ldg(row_zeros + g) : 0.0f;
@@ -636,7 +640,9 @@ scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       for (int column = w.s0 * kSlabK; column < end; column += kStepCols) {
         const int in_slot = column % kRawCols;
         const bool release = in_slot + kStepCols == kRawCols || column + kStepCols >= end;
-        if (S::kGroups == 2 && ((column / kStepCols) & 1) != group) {
+        const bool mine = S::kGroups == 1 || turn == group;
+        turn ^= 1;
+        if (!mine) {
           // the other group's stage; a last slot of nibbles with that stage alone is given back
           // by both groups
           if (kNibbles && release && in_slot == 0) {
@@ -648,8 +654,8 @@ scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           if (release) raw.advance(S::kRawSlots);
           continue;
         }
-        // (the stage first: that it is free says that everything up to three stages back has been
-        // consumed, so no barrier that is waited for here can be two phases behind)
+        // (the stage first: its last but one use is over, as this group has waited for that or for
+        // a later one, and that it is free says the same of the slots of packed codes)
         ok = mbar_wait_warp(&bars->empty[st.slot], st.phase ^ 1u, abort_flag);
         if (!ok) break;
         if (in_slot == 0 || S::kGroups == 2) {

@@ -37,6 +37,23 @@ def _tensor(qx, oracle_mod, rng, layout, group, n, k, act_order=None):
     return weights, oracle_mod.CanonicalTensor(layout, mode, n, k, group or k, data, scales, zeros, None, act_order)
 
 
+def _product_f64(tensor, x):
+    """The product in float64 by one matrix product: the oracle's loop takes seconds on large matrices."""
+    data = np.asarray(tensor.data).reshape(-1).view(np.uint8)
+    if tensor.layout == INT8:
+        q = data.view(np.int8).astype(np.float64)
+    else:
+        q = np.stack((data & 15, data >> 4), axis=-1).reshape(-1).astype(np.float64)
+        if tensor.layout == INT4:
+            q = np.where(q >= 8, q - 16, q)
+    q = q.reshape(tensor.rows, -1, tensor.group_size)
+    groups = (tensor.rows, q.shape[1], 1)
+    if tensor.zeros is not None:
+        q = q - np.asarray(tensor.zeros, np.float64).reshape(groups)
+    w = (q * np.asarray(tensor.scales, np.float64).reshape(groups)).reshape(tensor.rows, -1)
+    return x.astype(np.float64) @ w.T
+
+
 @pytest.mark.parametrize("layout,group,n,k,m,x_type", [
     (UINT4, 128, 4097, 2048, 5, BF16),   # smallest batch, a last tile of one row
     (UINT4, 128, 1025, 1152, 32, F16),   # half a slab at the end
@@ -63,6 +80,29 @@ def test_batches_against_float64(qx, orc, oracle_mod, layout, group, n, k, m, x_
     assert close(widen(typed, BF16), activation_f64(exact + bias.astype(np.float64)[None, :], 3), OUT_TOLERANCE[BF16])
     status, again = weights.qgemm_storage(x, x_type, m)  # pieces of a tile are added in a fixed order
     assert status == qx.OK and np.array_equal(again.view(np.uint32), y.view(np.uint32))
+    assert qx.lib.qx_check_device_errors() == qx.OK, qx.last_error()
+
+
+# Tiles that end on an odd number of 128-column stages, CTAs that go on to the next tile, rings of two
+# stages or two slots: f32 activations (three planes) of more than 32 tokens, bytes of 25 to 32
+@pytest.mark.parametrize("layout,group,n,k,m,x_type", [
+    (UINT4, 128, 4096, 4224, 64, F32),
+    (INT4, 64, 14336, 1152, 40, F32),
+    (INT8, 64, 12800, 1152, 28, F32),
+    (INT8, 128, 9000, 896, 60, F32),
+    (UINT4, 32, 25600, 96, 32, BF16),    # tiles of a single stage
+])
+def test_odd_stages_across_tiles(qx, orc, oracle_mod, layout, group, n, k, m, x_type):
+    rng = np.random.Generator(np.random.Philox(key=[n + k, m + group]))
+    weights, tensor = _tensor(qx, oracle_mod, rng, layout, group, n, k)
+    x, x_exact = _storage((rng.standard_normal((m, k)) * 0.1).astype(np.float32), x_type)
+    exact = _product_f64(tensor, x_exact)
+    status, first = weights.qgemm_storage(x, x_type, m)
+    assert status == qx.OK, qx.last_error()
+    assert close(first, exact)
+    for _ in range(5):
+        status, y = weights.qgemm_storage(x, x_type, m)
+        assert status == qx.OK and np.array_equal(y.view(np.uint32), first.view(np.uint32))
     assert qx.lib.qx_check_device_errors() == qx.OK, qx.last_error()
 
 

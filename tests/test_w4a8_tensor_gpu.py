@@ -64,6 +64,19 @@ def _twice_on_one_scratch(qx, packed, scales, x, m, n, k, fill=255):
     return results
 
 
+# Odd numbers of 128-column stages at the end of a tile, and CTAs that go on to the next tile behind
+# it: two groups of converter warps share rings of two stages (33 .. 64 rows that start on any byte)
+@pytest.mark.parametrize("m,n,k", [(33, 4096, 4098), (64, 14336, 1154), (48, 25600, 100), (40, 20000, 354)])
+def test_odd_stages_across_tiles(qx, orc, m, n, k):
+    rng = np.random.Generator(np.random.Philox(key=[m, n + k]))
+    packed = rng.integers(0, 256, (n, (k + 1) // 2), dtype=np.uint8)
+    scales = rng.uniform(0.001, 0.1, n).astype(np.float32)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    want = _exact(orc, packed, scales, x, m, n, k)
+    for y in _twice_on_one_scratch(qx, packed, scales, x, m, n, k):
+        assert np.array_equal(y.view(np.uint32), want.view(np.uint32))
+
+
 # tiles cut into pieces on a full grid, so that every CTA's counters are used: 16 epilogue warps
 # from 65 rows on, 8 below
 @pytest.mark.parametrize("m,n,k", [(64, 4096, 4096), (65, 4096, 4096), (100, 4096, 4098), (128, 14336, 4096)])
