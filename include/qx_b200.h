@@ -392,7 +392,8 @@ QX_API const char* qx_lowbit_gemm_variant(int format);
  * W4A8 for kInt4Row. Every activation row is quantised to int8 (quantize_int8 with one group
  * per row), the dot is an exact integer, Y = float(dot) * weight_scale[o] * activation_scale[r]
  * -- bit-identical to the reference. HOST pointers; the _dev form takes device pointers plus
- * qx_lowbit_w8a8_scratch_bytes(m, k) bytes of device scratch (it allocates nothing). */
+ * qx_lowbit_w8a8_scratch_bytes(m, k) bytes of device scratch (it allocates nothing). The size
+ * never falls as m or k grows: a scratch for the largest call serves every smaller one. */
 QX_API qx_status qx_lowbit_gemm_w8a8(const uint8_t* packed_weights, const float* weight_scales,
                               const float* x, float* y, long long m, long long n, long long k);
 QX_API size_t qx_lowbit_w8a8_scratch_bytes(long long m, long long k);

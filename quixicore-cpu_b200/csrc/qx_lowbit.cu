@@ -491,19 +491,24 @@ long long code_stride(long long k) { return (k + 7) / 8 * 8; }
 // tiles of more tokens are not cut into pieces (there are enough of them)
 constexpr long long kTensorPieceTokens = 128;
 size_t tensor_piece_bytes(long long m) {
-  if (m > kTensorPieceTokens) return 0;
   const long long tokens = m <= 64 ? (m + 31) / 32 * 32 : kTensorPieceTokens;
   return static_cast<size_t>(kTensorCtas) * 2 * 128 * tokens * sizeof(float);
 }
+constexpr long long kTensorMaxRows = 65535;
+// What any call of at most `m` rows and `k` columns uses: a scratch of one size serves all smaller
+// calls, so the pieces are counted where this call would have none, and the rows and columns up to
+// the limits of the tensor route.
 size_t tensor_scratch_bytes(long long m, long long k) {
-  return align_up(static_cast<size_t>(m) * code_stride(k) * 2, 256) + align_up(static_cast<size_t>(m) * 4, 256) +
-         align_up(kTensorCounterBytes, 256) + tensor_piece_bytes(m);
+  const size_t rows = static_cast<size_t>(m < kTensorMaxRows ? m : kTensorMaxRows);
+  const size_t row_bytes = static_cast<size_t>(code_stride(k < kTensorMaxK ? k : kTensorMaxK)) * 2;
+  return align_up(rows * row_bytes, 256) + align_up(rows * 4, 256) + align_up(kTensorCounterBytes, 256) +
+         tensor_piece_bytes(m);
 }
 // Where it is the faster one (us, here | dp4a kernel): rows on whole vectors, 4096 x 4096: 8 rows
 // 23.2 | 15.5, 16: 24.7 | 28.3, 64: 28 | 105; rows that start anywhere, 4096 x 4098: 4 rows
 // 21 | 78.8, 64: 29 | 1161; 2000 x 1502: 1 row 13 | 14.7, 4: 14 | 31.
 bool tensor_route(long long m, long long n, long long k) {
-  if (m > 65535 || n < 128 || k > kTensorMaxK) return false;
+  if (m > kTensorMaxRows || n < 128 || k > kTensorMaxK) return false;
   if (k % 32 != 0) return m >= 2 || n * k >= (1LL << 23);
   return m >= 13 || (m >= 5 && n * k >= (1LL << 25));
 }
@@ -651,11 +656,12 @@ qx_status qx_quantize_int8(const float* x, int8_t* codes, float* scales, long lo
 }
 
 // lowbit_gemm_w8a8 on the device: x f32 [m][k]; scratch_dev holds the activation codes,
-// scales and code sums: qx_lowbit_w8a8_scratch_bytes(m, k) bytes.
+// scales and code sums, or those in 16 bits with counters and pieces of tiles:
+// qx_lowbit_w8a8_scratch_bytes(m, k) bytes, never fewer for more rows or columns.
 size_t qx_lowbit_w8a8_scratch_bytes(long long m, long long k) {
   if (m <= 0 || k <= 0) return 0;
   const size_t codes = align_up(static_cast<size_t>(m) * k, 256) + 2 * align_up(static_cast<size_t>(m) * 4, 256);
-  const size_t tensor = m <= 65535 && k <= kTensorMaxK && (k % 32 != 0 || m >= 5) ? tensor_scratch_bytes(m, k) : 0;
+  const size_t tensor = tensor_scratch_bytes(m, k);
   return codes > tensor ? codes : tensor;
 }
 

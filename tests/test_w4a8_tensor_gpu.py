@@ -88,3 +88,24 @@ def test_pieces_of_a_full_grid(qx, orc, m, n, k):
     want = _exact(orc, packed, scales, x, m, n, k)
     for y in _twice_on_one_scratch(qx, packed, scales, x, m, n, k):
         assert np.array_equal(y.view(np.uint32), want.view(np.uint32))
+
+
+def test_scratch_of_the_largest_call_serves_smaller_ones(qx, orc):
+    import torch
+    n, guard = 4096, 32 << 20
+    size = int(qx.lib.qx_lowbit_w8a8_scratch_bytes(256, 4098))
+    scratch = torch.full((size + guard,), 0xA5, dtype=torch.uint8, device="cuda")
+    rng = np.random.Generator(np.random.Philox(key=[11, 12]))
+    for m, k in [(256, 4098), (128, 4096), (64, 4098), (5, 4096), (1, 2050)]:
+        packed = rng.integers(0, 256, (n, (k + 1) // 2), dtype=np.uint8)
+        scales = rng.uniform(0.001, 0.1, n).astype(np.float32)
+        x = rng.standard_normal((m, k)).astype(np.float32)
+        w, ws, xd = (torch.from_numpy(a).cuda() for a in (packed, scales, x))
+        y = torch.full((m, n), np.nan, device="cuda")
+        torch.cuda.synchronize()
+        status = qx.lib.qx_lowbit_gemm_w8a8_dev(w.data_ptr(), ws.data_ptr(), xd.data_ptr(), y.data_ptr(),
+                                                scratch.data_ptr(), m, n, k, torch.cuda.current_stream().cuda_stream)
+        assert status == qx.OK, qx.last_error()
+        torch.cuda.synchronize()
+        assert np.array_equal(y.cpu().numpy().view(np.uint32), _exact(orc, packed, scales, x, m, n, k).view(np.uint32))
+        assert bool((scratch[size:] == 0xA5).all())
