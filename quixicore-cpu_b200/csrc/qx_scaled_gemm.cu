@@ -11,7 +11,7 @@
 // over at most 128 columns, and the f32 scale is applied once per group by an f32 multiply-add
 // on the CUDA cores: no scale is ever rounded to 16 bits.
 //
-// Pipeline (persistent CTAs, one per SM, 24 or 28 warps):
+// Pipeline (persistent CTAs, one per SM, 28 warps):
 //   warp 0       packed codes: 16 KiB slots of [128 rows][128 bytes], 128-byte swizzled
 //                (256 columns of nibbles, 128 of bytes), by TMA or, from a panel, bulk copies
 //   warp 2       activations: TMA tiles of bn tokens x 64 columns, into the stage's B part
@@ -19,8 +19,8 @@
 //   warp 1       MMA issuer: one wait and one commit per stage (128 columns, all planes),
 //                8 x tcgen05.mma per plane; a new accumulator every `promote` columns (32 / 64 /
 //                128: what the group size allows)
-//   epilogue     thread = weight row: tcgen05.ld, acc += scale * partial (packed f32x2 FMAs);
-//                at the end bias, activation, store
+//   epilogue     thread = weight row: tcgen05.ld, acc += scale * partial (packed f32x2 FMAs), every
+//                8 or 16 of them into totals in TMEM; at the end bias, activation, store
 // What bounds it is less the tensor core than the chains of single instructions around it: a
 // successful barrier wait costs about 80 cycles, a commit 30, a pair of MMAs 100 or more, so a
 // step of 64 columns with four waits and three commits took 1300 cycles where its MMAs (32
@@ -60,10 +60,15 @@ constexpr int kMaxStages = 3, kMaxRaw = 4, kMaxAcc = 4;
 constexpr int kFinishCols = 16;            // columns an epilogue warp finishes at a time
 constexpr size_t kSmemMax = 227 * 1024;
 constexpr int kTmemCols = 512;             // all of it: one CTA per SM
+// Scaled units in a row of f32 multiply-adds: rows of many units may take longer chains, as the digit
+// kernels' own error grows with the row (q8_0: 6.6e-8 of the result at 32 units, 9.0e-8 at 256,
+// 9.6e-8 at 344; chains of 8 are worth 6.2e-8 and chains of 16 8.0e-8 at any length).
+constexpr int kChain = 8, kLongChain = 16, kLongRowUnits = 256;
 
 // EPI epilogue warps, CONV converter warps, COLS accumulator columns of an epilogue warp at most.
 // Registers per thread of the warpgroups (issue warps, epilogue, converters): they add up to at
-// most what the block is launched with (checked against the compiled kernel in launch_kernel).
+// most what the block is launched with (checked against the compiled kernel in launch_kernel). With
+// 32 for the issue warps the MMA thread spills (16 tokens on 14336 x 4096 uint4: 35.2 us against 31.6).
 template <int EPI_, int CONV_, int COLS_, int RAW_, int R_ISSUE, int R_EPI, int R_CONV>
 struct Shape {
   static constexpr int kEpi = EPI_, kConv = CONV_, kCols = COLS_, kRawSlots = RAW_;
@@ -73,12 +78,13 @@ struct Shape {
   static constexpr int kRegShares = R_ISSUE + EPI_ / 4 * R_EPI + CONV_ / 4 * R_CONV;
   static constexpr int kTokens = COLS_ * (EPI_ / 4);  // per tile at most
   static constexpr int kFinishBytes = EPI_ * 32 * kFinishCols * 4;
+  static_assert(COLS_ == 32, "an epilogue warp reads the columns of a unit at once");
   static_assert(RAW_ <= kMaxRaw && EPI_ <= kScaledEpilogueWarps && CONV_ % 8 == 0 &&
                     65536 / kThreads / 8 * 8 * (kThreads / 128) >= kRegShares, "shape");
 };
-using Small = Shape<8, 16, 32, 4, 32, 120, 56>;
-using SmallPlanes = Shape<8, 16, 32, 2, 32, 120, 56>;  // three planes: larger stages
-using Large = Shape<16, 8, 32, 3, 32, 88, 56>;
+using Small = Shape<8, 16, 32, 4, 40, 104, 56>;
+using SmallPlanes = Shape<8, 16, 32, 2, 40, 104, 56>;  // three planes: larger stages
+using Large = Shape<16, 8, 32, 3, 40, 88, 56>;
 
 struct ScaledParams {
   const uint8_t* panel;
@@ -96,8 +102,9 @@ struct ScaledParams {
   int columns;                 // rounded up to whole stages
   int slabs, bn, stages;
   int promote, promote_log;    // columns per accumulator
-  int hand_cols;               // columns per hand-over to the epilogue: max(promote, a stage's)
+  int hand_cols;               // columns per hand-over to the epilogue: promote .. a stage's
   int accs;                    // hand-overs in flight in TMEM
+  int chain;                   // units per chain
   int o_tiles, r_tiles, split, y_type, activation;
 };
 
@@ -347,7 +354,7 @@ scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
           for (int h = 0; h < 2 * kSubs; ++h) {  // 32 columns
             const uint32_t at = (column + 32 * h) & hand_mask;
-            if ((h & 1) == 0 && at == 0) {  // (hand-overs start on multiples of 64 columns)
+            if (at == 0) {
               ok = mbar_wait(&bars->tmem_empty[acc.slot], acc.phase ^ 1u, abort_flag);
               if (!ok) break;
               tc_fence_after_sync();
@@ -355,7 +362,7 @@ scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             const uint32_t d = tmem_base + acc.slot * hand_size + (at >> promote_log) * bn;
             uint32_t started = (at & promote_mask) != 0 ? 1u : 0u;
 #pragma unroll
-            for (int plane = 0; plane < PLANES; ++plane) {
+            for (int plane = PLANES - 1; plane >= 0; --plane) {  // (the small parts first)
               // 16 columns = 32 bytes inside the swizzle atom: +2 in the (address >> 4) field
               const uint64_t ad = a_desc + (h >> 1) * (kABytes >> 4) + 4 * (h & 1);
               const uint64_t bd = b_desc + ((h >> 1) * PLANES + plane) * b_units + 4 * (h & 1);
@@ -363,7 +370,7 @@ scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
               mma_f16_ss(d, ad + 2, bd + 2, idesc, 1u);
               started = 1u;
             }
-            if ((h & 1) == 1 && at + 32 == static_cast<uint32_t>(p.hand_cols)) {
+            if (at + 32 == static_cast<uint32_t>(p.hand_cols)) {
               tc_commit(&bars->tmem_full[acc.slot]);
               acc.advance(p.accs);
             }
@@ -384,6 +391,7 @@ scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int cols = p.bn / (S::kEpi / 4);  // columns of this warp
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                                static_cast<uint32_t>(half * cols);
+    const uint32_t total_base = lane_base + static_cast<uint32_t>(kTmemCols - 2 * p.bn);
     const uint32_t hand_size = static_cast<uint32_t>(p.bn) << (31 - __clz(p.hand_cols) - p.promote_log);
     float* my_finish = finish + (warp - 4) * 32 * kFinishCols + lane;
     Ring acc;
@@ -394,120 +402,150 @@ scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       unsigned long long sum[S::kCols / 2];
 #pragma unroll
       for (int i = 0; i < S::kCols / 2; ++i) sum[i] = 0ull;
-      // Two levels of f32 sums: 32 units at a time, then those into `total` (local memory: it is
-      // touched once per 32 units and the registers are full). One chain over all units of a long
-      // row would show its roundings (q8_0, 11008 columns: 2.4e-7 of the result, 1.1e-7 with two
-      // levels, which is where the digit kernels are); every eight units would cost more than it
-      // gives (331 tokens on 4096 x 11008: 275 us).
-      volatile float total[S::kCols];
+      // Two levels of sums: chains of multiply-adds in registers, then each chain into a total and
+      // what the total's roundings lost, both in TMEM columns behind the accumulators. So a result
+      // is one chain's few roundings away from exact whatever the length of the row, and no
+      // further than the separate lanes of the digit kernels leave it (q8_0, 11008 columns: 8.4e-8
+      // of the result, digit kernels 9.6e-8, one chain over all units 2.4e-7; 1024 columns: 6.2e-8
+      // and 6.6e-8). Whole numbers (W4A8) are exact in one chain. Not in registers or local
+      // memory: the former are full, the latter has next to no L1 beside the shared memory.
+      // A total costs 4 % of 512 tokens on 14336 x 4096 uint4, 11 % of 331 on 4096 x 11008 q8_0.
       bool flushed = false;
-      int pending = 0;
-      const int begin = w.s0 * kSlabK;
-      const int end = min(w.s1 * kSlabK, p.columns);
-      // scale of the unit at `column`, fetched one group (panel: one slab) ahead
-      const float* row_scales = p.scales + static_cast<long long>(live ? row : 0) * p.groups;
-      int g = SRC == kScaledPanelQ8 ? 0 : begin / p.group;
-      int boundary = (g + 1) * p.group;
-      const uint8_t* panel_scales = p.panel + (static_cast<long long>(o_tile) * p.slabs) * slab_span_bytes(QX_FORMAT_Q8_0) +
-                                    panel_scale_offset(QX_FORMAT_Q8_0, quarter * 32 + lane, 0);
-      uint4 block_scales = make_uint4(0u, 0u, 0u, 0u), next_blocks = block_scales;
-      float scale = 0.0f, next_scale = 0.0f;
-      if (SRC == kScaledPanelQ8) {
-        next_blocks = __ldg(reinterpret_cast<const uint4*>(panel_scales + static_cast<long long>(w.s0) * slab_span_bytes(QX_FORMAT_Q8_0)));
-      } else if (p.token_scales != nullptr) {
-        scale = next_scale = 1.0f;  // whole numbers are summed; the scales come at the end
-      } else {
-        scale = live ? __ldg(row_scales + g) : 0.0f;
-        next_scale = live && g + 1 < p.groups ? __ldg(row_scales + g + 1) : 0.0f;
-      }
-      for (int column = begin; column < end; column += p.hand_cols) {
-        if (SRC == kScaledPanelQ8 && column % kSlabK == 0) {
-          block_scales = next_blocks;
-          const int s = column / kSlabK + 1;
-          if (s < w.s1) {
-            next_blocks = __ldg(reinterpret_cast<const uint4*>(panel_scales + static_cast<long long>(s) * slab_span_bytes(QX_FORMAT_Q8_0)));
+      auto flush = [&]() {
+        if (flushed) tmem_st_wait();
+#pragma unroll
+        for (int c = 0; c < S::kCols; c += 8) {  // (few columns at a time: the registers are full)
+          if (c >= cols) break;
+          uint32_t total[8], rest[8];
+          if (flushed) {
+            tmem_ld_32x8(total_base + c, total);
+            tmem_ld_32x8(total_base + p.bn + c, rest);
+            tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) total[i] = rest[i] = 0u;
           }
+#pragma unroll
+          for (int i = 0; i < 8; i += 2) {
+            unsigned long long t = pack2(total[i], total[i + 1]), r = pack2(rest[i], rest[i + 1]);
+            add_with_rest2(t, r, sum[(c + i) / 2]);
+            sum[(c + i) / 2] = 0ull;
+            unpack2(t, total[i], total[i + 1]);
+            unpack2(r, rest[i], rest[i + 1]);
+          }
+          tmem_st_32x8(total_base + c, total);
+          tmem_st_32x8(total_base + p.bn + c, rest);
         }
+        flushed = true;
+      };
+      // Waits for the accumulators of the next hand-over; false when the kernel gives up.
+      auto take = [&]() {
         ok = mbar_wait_warp(&bars->tmem_full[acc.slot], acc.phase, abort_flag);
-        if (!ok) break;
         tc_fence_after_sync();
-        uint32_t taddr = lane_base + acc.slot * hand_size;
-        const int hand_end = min(column + p.hand_cols, end);
-        for (int unit = column; unit < hand_end; unit += p.promote, taddr += p.bn) {
-          if (SRC == kScaledPanelQ8) {
-            const int block = (unit / 32) % kSlabBlocks;
-            const uint32_t lo = (block & 4) ? block_scales.z : block_scales.x;
-            const uint32_t hi = (block & 4) ? block_scales.w : block_scales.y;
-            const uint32_t both = (block & 2) ? hi : lo;
-            scale = half_bits_to_float(static_cast<unsigned short>((block & 1) ? both >> 16 : both));
-          } else if (unit >= boundary) {
-            scale = next_scale;  // (0 past the last group: padding columns of the last stage)
-            ++g;
-            boundary += p.group;
-            next_scale = live && g + 1 < p.groups ? __ldg(row_scales + g + 1) : 0.0f;
-          }
-          const uint32_t s_bits = __float_as_uint(scale);
-          const unsigned long long s2 = pack2(s_bits, s_bits);
-          const bool last_unit = unit + p.promote >= hand_end;
-          // 32 columns at a time, the next ones on their way while these are added
-          uint32_t v[2][32];
-          if (cols >= 32) {
-            tmem_ld_32x32(taddr, v[0]);
-          } else {  // (32 tokens per tile: 16 columns each)
-            tmem_ld_32x16_low(taddr, v[0]);
-          }
+        return ok;
+      };
+      // sum += scale * accumulators at `taddr`; `release`: the last ones of the hand-over.
+      // 16 columns at a time: with 32 of them in registers the loop spills (q8_0, 331 tokens on
+      // 4096 x 11008: 147 us against 139).
+      auto add_unit = [&](uint32_t taddr, float scale, bool release) {
+        const unsigned long long s2 = pack2(__float_as_uint(scale), __float_as_uint(scale));
+#pragma unroll
+        for (int c = 0; c < S::kCols; c += 16) {
+          if (c >= cols) break;
+          uint32_t v[16];
+          tmem_ld_32x16(taddr + c, v);
           tmem_ld_wait();
-#pragma unroll
-          for (int c = 0; c < S::kCols; c += 32) {
-            const bool more = c + 32 < S::kCols && c + 32 < cols;
-            if (more) tmem_ld_32x32(taddr + c + 32, v[(c / 32 + 1) & 1]);
-            if (last_unit && !more && c < cols) {
-              tc_fence_before_sync();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&bars->tmem_empty[acc.slot]);
-            }
-            if (c < cols) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                fma2(sum[c / 2 + j], pack2(v[(c / 32) & 1][2 * j], v[(c / 32) & 1][2 * j + 1]), s2);
-              }
-            }
-            if (more) tmem_ld_wait();
+          if (release && c + 16 >= cols) {
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->tmem_empty[acc.slot]);
           }
-          if (++pending == 32 && unit + p.promote < end) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) fma2(sum[c / 2 + j], pack2(v[2 * j], v[2 * j + 1]), s2);
+        }
+      };
+      const float* row_scales = p.scales + static_cast<long long>(live ? row : 0) * p.groups;
+      if (SRC == kScaledPanelQ8) {
+        // scales come one slab (eight units) ahead; a chain is one slab, or two
+        const int hand_units = S::kEpi == 16 ? 1 : p.hand_cols / 32;
+        int pending = 0;
+        const uint8_t* slab_scales = p.panel + (static_cast<long long>(o_tile) * p.slabs + w.s0) * slab_span_bytes(QX_FORMAT_Q8_0) +
+                                     panel_scale_offset(QX_FORMAT_Q8_0, quarter * 32 + lane, 0);
+        uint4 next = __ldg(reinterpret_cast<const uint4*>(slab_scales));
+        for (int s = w.s0; s < w.s1 && ok; ++s) {
+          uint4 blocks = next;
+          slab_scales += slab_span_bytes(QX_FORMAT_Q8_0);
+          if (s + 1 < w.s1) next = __ldg(reinterpret_cast<const uint4*>(slab_scales));
+          const int units = min(kSlabK, p.columns - s * kSlabK) / 32;
+          for (int u = 0; u < units; ++u) {
+            const int at = u & (hand_units - 1);
+            if (at == 0 && !take()) break;
+            const bool last = at == hand_units - 1;
+            add_unit(lane_base + acc.slot * hand_size + at * p.bn,
+                     half_bits_to_float(static_cast<unsigned short>(blocks.x)), last);
+            if (last) acc.advance(p.accs);
+            blocks.x = __funnelshift_r(blocks.x, blocks.y, 16);
+            blocks.y = __funnelshift_r(blocks.y, blocks.z, 16);
+            blocks.z = __funnelshift_r(blocks.z, blocks.w, 16);
+            blocks.w >>= 16;
+          }
+          pending += kSlabK / 32;
+          if (pending == p.chain && s + 1 < w.s1) {
             pending = 0;
-            float t[S::kCols];  // (all reads before the first write: they overlap)
-#pragma unroll
-            for (int i = 0; i < S::kCols; ++i) t[i] = flushed ? total[i] : 0.0f;
-#pragma unroll
-            for (int i = 0; i < S::kCols / 2; ++i) {
-              float v0, v1;
-              unpack2(sum[i], v0, v1);
-              total[2 * i] = t[2 * i] + v0;
-              total[2 * i + 1] = t[2 * i + 1] + v1;
-              sum[i] = 0ull;
-            }
-            flushed = true;
+            flush();
           }
         }
-        acc.advance(p.accs);
+      } else {
+        const int begin = w.s0 * kSlabK;
+        const int end = min(w.s1 * kSlabK, p.columns);
+        const int hand_units = p.hand_cols >> p.promote_log;
+        int pending = 0;
+        // scale of the unit at `column`, fetched one group ahead
+        int g = begin / p.group;
+        int boundary = (g + 1) * p.group;
+        float scale = 1.0f, next_scale = 1.0f;
+        if (p.token_scales == nullptr) {  // (whole numbers are summed; the scales come at the end)
+          scale = live ? __ldg(row_scales + g) : 0.0f;
+          next_scale = live && g + 1 < p.groups ? __ldg(row_scales + g + 1) : 0.0f;
+        }
+        for (int column = begin; column < end; column += p.hand_cols) {
+          if (!take()) break;
+          uint32_t taddr = lane_base + acc.slot * hand_size;
+          const int hand_end = min(column + p.hand_cols, end);
+          for (int unit = column; unit < hand_end; unit += p.promote, taddr += p.bn) {
+            if (unit >= boundary) {
+              scale = next_scale;  // (0 past the last group: padding columns of the last stage)
+              ++g;
+              boundary += p.group;
+              next_scale = live && g + 1 < p.groups ? __ldg(row_scales + g + 1) : 0.0f;
+            }
+            add_unit(taddr, scale, unit + p.promote >= hand_end);
+          }
+          acc.advance(p.accs);
+          pending += hand_units;  // (1, 2 or 4)
+          if (pending == p.chain && column + p.hand_cols < end && p.token_scales == nullptr) {
+            pending = 0;
+            flush();
+          }
+        }
       }
       if (!ok) break;
-      if (flushed) {
-        float t[S::kCols];
+      flush();
+      tmem_st_wait();
+      // Finish the tile, kFinishCols columns at a time in ROLLED loops: this code runs once per
+      // tile, and unrolled it costs more in instruction fetches than in work. A piece of a tile
+      // goes to scratch; whoever completes the tile's count adds the pieces in CTA order.
+      auto finished = [&](int c, float (&out)[kFinishCols]) {
+        uint32_t total[kFinishCols], rest[kFinishCols];
+        tmem_ld_32x16(total_base + c, total);
+        tmem_ld_32x16(total_base + p.bn + c, rest);
+        tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < S::kCols; ++i) t[i] = total[i];
-#pragma unroll
-        for (int i = 0; i < S::kCols / 2; ++i) {
-          float v0, v1;
-          unpack2(sum[i], v0, v1);
-          sum[i] = pack2(__float_as_uint(t[2 * i] + v0), __float_as_uint(t[2 * i + 1] + v1));
+        for (int i = 0; i < kFinishCols; ++i) {  // (a total that is not finite has no rest)
+          const float t = __uint_as_float(total[i]);
+          out[i] = isfinite(t) ? t + __uint_as_float(rest[i]) : t;
         }
-      }
-      // Finish the tile, kFinishCols columns at a time in ROLLED loops (the accumulators move
-      // down by one chunk per turn): this code runs once per tile, and unrolled it costs more
-      // in instruction fetches than in work. A piece of a tile goes to scratch; whoever
-      // completes the tile's count adds the pieces in CTA order.
+      };
       const size_t slot_floats = static_cast<size_t>(kRows) * p.bn;
       const size_t mine = static_cast<size_t>(half * cols) * kRows + quarter * 32 + lane;
       const bool piece = p.split && !(w.s0 == 0 && w.s1 == p.slabs);
@@ -527,16 +565,11 @@ scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         float* own = piece_of(blockIdx.x);
 #pragma unroll 1
         for (int c = 0; c < tokens; c += kFinishCols) {
+          float part[kFinishCols];
+          finished(c, part);
 #pragma unroll
-          for (int i = 0; i < kFinishCols / 2; ++i) {
-            float v0, v1;
-            unpack2(sum[i], v0, v1);
-            __stcg(own + (2 * i) * kRows, v0);
-            __stcg(own + (2 * i + 1) * kRows, v1);
-          }
+          for (int i = 0; i < kFinishCols; ++i) __stcg(own + i * kRows, part[i]);
           own += kFinishCols * kRows;
-#pragma unroll
-          for (int i = 0; i + kFinishCols / 2 < S::kCols / 2; ++i) sum[i] = sum[i + kFinishCols / 2];
         }
         __threadfence();
         __syncwarp();
@@ -551,36 +584,28 @@ scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         __threadfence();
       }
       const float bias = p.bias != nullptr && live ? __ldg(p.bias + row) : 0.0f;
-      if (piece) {
-#pragma unroll
-        for (int i = 0; i < S::kCols / 2; ++i) sum[i] = 0ull;
-        for (int k = c0; k <= c1; ++k) {  // (all columns of a piece at once: the reads overlap)
-          const float* in = piece_of(k);
-#pragma unroll
-          for (int i = 0; i < S::kCols / 2; ++i) {
-            if (2 * i < tokens) {
-              float v0, v1;
-              unpack2(sum[i], v0, v1);
-              v0 += __ldcg(in + (2 * i) * kRows);
-              v1 += __ldcg(in + (2 * i + 1) * kRows);
-              sum[i] = pack2(__float_as_uint(v0), __float_as_uint(v1));
-            }
-          }
-        }
-      }
       const float row_scale = p.token_scales != nullptr && live ? __ldg(row_scales) : 1.0f;
       long long at = token0 * p.ldy + row;
 #pragma unroll 1
       for (int c = 0; c < tokens; c += kFinishCols) {
+        if (piece) {  // (in 64 bits: a piece adds no rounding but its own)
+          double whole[kFinishCols];
 #pragma unroll
-        for (int i = 0; i < kFinishCols / 2; ++i) {
-          float v0, v1;
-          unpack2(sum[i], v0, v1);
-          my_finish[(2 * i) * 32] = v0;
-          my_finish[(2 * i + 1) * 32] = v1;
+          for (int i = 0; i < kFinishCols; ++i) whole[i] = 0.0;
+#pragma unroll 2
+          for (int k = c0; k <= c1; ++k) {
+            const float* in = piece_of(k) + c * kRows;
+#pragma unroll
+            for (int i = 0; i < kFinishCols; ++i) whole[i] += __ldcg(in + i * kRows);
+          }
+#pragma unroll
+          for (int i = 0; i < kFinishCols; ++i) my_finish[i * 32] = static_cast<float>(whole[i]);
+        } else {
+          float part[kFinishCols];
+          finished(c, part);
+#pragma unroll
+          for (int i = 0; i < kFinishCols; ++i) my_finish[i * 32] = part[i];
         }
-#pragma unroll
-        for (int i = 0; i + kFinishCols / 2 < S::kCols / 2; ++i) sum[i] = sum[i + kFinishCols / 2];
         const int count = tokens - c < kFinishCols ? tokens - c : kFinishCols;
         if (live) {
 #pragma unroll 4
@@ -797,10 +822,13 @@ Plan make_plan(const ScaledGemmArgs& a, int sm_count) {
   p.staged = p.planes == 3 || a.order != nullptr || reinterpret_cast<uintptr_t>(a.x) % 16 != 0;
   p.staged_bytes = p.staged ? align_up(static_cast<size_t>(p.planes) * a.m * a.columns * 2, 256) : 0;
   p.promote = a.group % 128 == 0 || a.group == a.columns ? 128 : (a.group % 64 == 0 ? 64 : 32);
-  // Three planes: the sums of 32 columns leave the tensor core, or its own f32 adds would show
-  // (4096 columns, scale groups of 128: 4.9e-7 of the result after 128 columns each, 2.2e-7
-  // after 32, with the digit kernels at 2.4e-7).
-  if (p.planes == 3) p.promote = 32;
+  // Three planes: the sums of 64 columns leave the tensor core, or its own f32 adds would show
+  // (scale groups of 128: 3.2e-7 of the result after 128 columns each, 1.5e-7 after 64, digit
+  // kernels 2.3e-7 to 2.5e-7; bytes 3.5e-7 and 1.7e-7). And f16 activations on bytes, products of
+  // 18 bits, those of 32 columns (groups of 128: 1.2e-7 after 128 columns, 7.5e-8 after 32, digit
+  // kernels 7.0e-8 to 9.8e-8).
+  if (p.planes == 3 && p.promote > 64) p.promote = 64;
+  if (a.source == kScaledBytes && a.x_type == QX_STORAGE_F16) p.promote = 32;
   p.small = a.m <= Small::kTokens || p.planes == 3;  // (three planes of 128 tokens: no two stages)
   const int most = p.small ? Small::kTokens : Large::kTokens;
   p.r_tiles = static_cast<int>((a.m + most - 1) / most);
@@ -829,11 +857,15 @@ qx_status launch_kernel(const CUtensorMap& map_w, const CUtensorMap& map_x, Scal
                         cudaStream_t stream) {
   p.stages = stages_for<S>(p.bn, PLANES, raw_bytes(SRC));
   p.promote_log = p.promote == 128 ? 7 : (p.promote == 64 ? 6 : 5);
-  // one hand-over of accumulators per stage, two where four of them would fill TMEM
-  p.hand_cols = p.promote == 32 && p.bn > 64 ? 64 : kStepCols;
+  // one hand-over of accumulators per stage, or shorter ones where two would not fit beside the
+  // totals and their rests
+  const int free_cols = kTmemCols - 2 * p.bn;
+  p.hand_cols = kStepCols;
+  while (p.hand_cols > p.promote && 2 * p.bn * (p.hand_cols / p.promote) > free_cols) p.hand_cols /= 2;
   const int hand = p.bn * (p.hand_cols / p.promote);
-  p.accs = kTmemCols / hand > kMaxAcc ? kMaxAcc : kTmemCols / hand;
-  if (p.accs < 1) {
+  p.accs = free_cols / hand > kMaxAcc ? kMaxAcc : free_cols / hand;
+  p.chain = p.columns >> p.promote_log >= kLongRowUnits ? kLongChain : kChain;
+  if (p.accs < 2 || (SRC == kScaledPanelQ8 && S::kEpi == 16 && p.hand_cols != 32)) {
     set_last_error_text("scaled projection: accumulators beyond TMEM");
     return QX_STATUS_DEVICE_ERROR;
   }

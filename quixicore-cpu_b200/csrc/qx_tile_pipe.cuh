@@ -37,14 +37,30 @@ __device__ __forceinline__ unsigned long long pack2(uint32_t lo, uint32_t hi) {
   asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
   return v;
 }
-__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
-  uint32_t a, b;
-  asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(v));
-  lo = __uint_as_float(a);
-  hi = __uint_as_float(b);
+__device__ __forceinline__ void unpack2(unsigned long long v, uint32_t& lo, uint32_t& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
 }
 __device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+__device__ __forceinline__ unsigned long long addf2(unsigned long long a, unsigned long long b) {
+  unsigned long long v;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
+__device__ __forceinline__ unsigned long long subf2(unsigned long long a, unsigned long long b) {
+  unsigned long long v;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
+// total += value; what the rounding of that lost goes to `rest` (Dekker's fast two-sum: exact where
+// the total is the larger one, as it is of a sum of many, and at worst one more rounding of a value)
+__device__ __forceinline__ void add_with_rest2(unsigned long long& total, unsigned long long& rest,
+                                               unsigned long long value) {
+  const unsigned long long sum = addf2(total, value);
+  rest = addf2(rest, subf2(value, subf2(sum, total)));
+  total = sum;
 }
 
 // ---- 16-bit whole numbers ----------------------------------------------------------------
