@@ -998,11 +998,16 @@ qx_status launch_any(const CanonicalParams& p, bool digits, uint32_t* image, int
 }
 
 // Which batches take the tensor cores with scales applied per group (qx_scaled_gemm.cu).
-// Measured there | here (us, bf16 tokens unless noted):
-//   uint4, groups of 128, 14336 x 4096:  4 tokens 32.9 | 36.7,  5: 33.5 | 61.7,  512: 138 | 3596
-//   4096 x 4096:  4 tokens 18.2 | 16.9,  5: 19.3 | 26.8,  128: 30 | 272
-//   f32 activations (three planes), groups of 32, 14336 x 4096: 25 tokens 66.7 | 200;
-//   1024 x 1024: 32 tokens 15.7 | 13.3,  64: 17.9 | 19.2
+// Measured there | on the digit kernels (us; `work` = tokens x rows x columns):
+//   groups of 64 and more, 16-bit tokens (uint4, groups of 128), from 1024 rows on:
+//     1024 x 1024: 32 tokens 11.9 | 13.5;  2048 x 2048: 8: 13.6 | 11.0,  16: 14.4 | 18.2;
+//     4096 x 4096: 5: 18.0 | 24.2,  128: 33 | 271;  14336 x 4096: 5: 31.0 | 63.9
+//   4-bit groups of 32, where a unit is 32 columns and the digit kernels are at their best:
+//     2048 x 2048: 16 tokens 15.3 | 13.9,  32: 15.7 | 23.0;  4096 x 4096: 8: 22.6 | 20.9,  16: 23.4 | 36.3
+//   fewer rows (few tiles, many pieces): 512 x 2048, 32 tokens 14.4 | 11.8,  64: 22.7 | 19.5,  128: 26.3 | 28.8
+//   long rows (few warps on the digit kernels): 1024 x 8192, 5 tokens 21.6 | 26.9, groups of 32 23.0 | 25.6
+//   f32 tokens (three planes): 1024 x 1024, 64 tokens 19.5 | 19.5;  2048 x 2048, 25: 17.7 | 22.6;
+//     14336 x 4096, 25: 44 | 202
 // int8 with one scale per row stays on the digit planes below, whose sums over the whole row are
 // exact: f32 sums of the tensor core over 128 columns are 1.6 to 3.3 times as far from float64
 // (512 f16 tokens, 4096 x 4096: 1.5e-7 against 4.5e-8 of the result).
@@ -1011,9 +1016,20 @@ bool scaled_route(const qx_canonical_weights* w, int x_type, long long m) {
   if (w->group_index != nullptr || w->rows < 128) return false;
   // fractional zero points have no exact 16-bit form
   if (w->layout == QX_CANONICAL_UINT4_AFFINE && !w->integral_zeros) return false;
-  const long long work = m * w->rows * w->columns;
   if (w->layout == QX_CANONICAL_INT8_SYMMETRIC && w->groups_per_row == 1) return false;
-  return x_type == QX_STORAGE_F32 ? m >= 25 && work >= (1LL << 26) : m >= 5 && work >= (1LL << 25);
+  const bool f32 = x_type == QX_STORAGE_F32;
+  const bool narrow = w->layout != QX_CANONICAL_INT8_SYMMETRIC && w->groups_per_row > 1 && w->group_size % 64 != 0;
+  long long least;
+  if (w->rows >= 1024 && w->columns >= 8192 && !f32) {
+    least = 1LL << 25;
+  } else if (narrow || w->rows < 1024) {
+    least = (1LL << 27) + (narrow ? 1 : 0);
+  } else if (f32) {
+    least = 3LL << 25;
+  } else {
+    least = m >= 16 ? 1LL << 25 : 1LL << 26;
+  }
+  return m >= (f32 ? 25 : 5) && m * w->rows * w->columns >= least;
 }
 
 qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_type,

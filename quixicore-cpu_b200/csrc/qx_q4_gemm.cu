@@ -24,7 +24,7 @@
 // (relative error at most 2^-12 per weight); products are exact and sums f32 in the tensor
 // core. This is the stated 1e-2 tolerance class of the 4-bit prefill path (measured: about
 // 2e-4 of a row's rms); batches below 64 rows take the exact digit kernels instead, and q8_0
-// weights those or, from 16 rows on, the scaled-projection kernel (qx_scaled_gemm.cu).
+// weights those or, from 16 or 17 rows on, the scaled-projection kernel (qx_scaled_gemm.cu).
 
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -357,10 +357,14 @@ q4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const Q4GemmParams 
   }
 }
 
-// q8_0 panels take the scaled-projection kernel (qx_scaled_gemm.cu) from this many tokens on:
-// 14336 x 4096, 16 tokens 37.5 us against 39.0 on the digit kernels, 24: 37.9 against 62.1;
-// 4096 x 11008, 16 tokens 34.1 against 35.9, 331: 130 against 664.
-constexpr long long kScaledPrefillRows = 16;
+// q8_0 panels take the scaled-projection kernel (qx_scaled_gemm.cu) from 17 tokens on, which the
+// digit kernels cut into two launches, and with 16 on matrices of at most 2^24 weights. Measured
+// there | on the digit kernels (us): 16 tokens: 1024 x 1024 12.1 | 18.8, 4096 x 4096 22.8 | 25.5, 4096 x 11008
+// 38.3 | 37.0, 14336 x 4096 45.5 | 39.3;  17: 14336 x 4096 45.9 | 56.4, 28672 x 8192 138 | 160;
+// 331: 4096 x 11008 139 | 664.
+bool scaled_prefill(const qx_weights* w, long long m) {
+  return m >= 17 || (m == 16 && w->rows * w->columns <= (1LL << 24));
+}
 
 constexpr size_t kQ4GemmSmem = 1024 + kASlots * kABytes + kBSlots * kMaxTokens * 128 +
                                kRawSlots * kRawBytes + sizeof(Q4GemmBarriers) + 64;
@@ -461,7 +465,7 @@ qx_status launch_q4_gemm_bf16(const qx_weights* w, const uint16_t* x_bf16_dev, f
       m * w->columns < (1LL << 40)) {
     return launch_tc(w, x_bf16_dev, y_dev, m, ldy, ws, stream);
   }
-  if (w->format == QX_FORMAT_Q8_0 && w->segments == 1 && m >= kScaledPrefillRows) {
+  if (w->format == QX_FORMAT_Q8_0 && w->segments == 1 && scaled_prefill(w, m)) {
     ScaledGemmArgs a{};
     a.source = kScaledPanelQ8;
     a.codes = w->panel;

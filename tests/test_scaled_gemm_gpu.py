@@ -83,6 +83,31 @@ def test_batches_against_float64(qx, orc, oracle_mod, layout, group, n, k, m, x_
     assert qx.lib.qx_check_device_errors() == qx.OK, qx.last_error()
 
 
+# The same edges above the lines at which the tensor cores take over
+@pytest.mark.parametrize("layout,group,n,k,m,x_type", [
+    (UINT4, 128, 4097, 4096, 5, BF16),   # smallest batch, a last tile of one row
+    (INT4, 32, 4001, 1056, 33, BF16),    # 33 groups: the last stage holds groups of padding
+    (UINT4, 32, 2300, 992, 64, F32),     # three planes, largest small tile
+    (INT4, 64, 1030, 2112, 65, F16),     # first large tile
+    (UINT4, 96, 1010, 1152, 130, BF16),  # groups that do not divide a slab
+    (INT4, 0, 700, 800, 257, F32),       # one scale per row, tokens in five tiles
+    (UINT4, 128, 130, 8192, 128, F16),   # two tiles in pieces of one slab each
+    (INT8, 64, 2000, 1088, 70, F32),     # bytes: half a slot at the end
+    (UINT4, 128, 14336, 1024, 512, BF16),  # several rounds of tiles on every SM
+])
+def test_edges_above_the_lines(qx, orc, oracle_mod, layout, group, n, k, m, x_type):
+    rng = np.random.Generator(np.random.Philox(key=[n * 31 + k, m * 7 + group]))
+    weights, tensor = _tensor(qx, oracle_mod, rng, layout, group, n, k)
+    x, x_exact = _storage((rng.standard_normal((m, k)) * 0.1).astype(np.float32), x_type)
+    exact = _product_f64(tensor, x_exact)
+    status, y = weights.qgemm_storage(x, x_type, m)
+    assert status == qx.OK, qx.last_error()
+    assert close(y, exact)
+    status, again = weights.qgemm_storage(x, x_type, m)
+    assert status == qx.OK and np.array_equal(again.view(np.uint32), y.view(np.uint32))
+    assert qx.lib.qx_check_device_errors() == qx.OK, qx.last_error()
+
+
 # Tiles that end on an odd number of 128-column stages, CTAs that go on to the next tile, rings of two
 # stages or two slots: f32 activations (three planes) of more than 32 tokens, bytes of 25 to 32
 @pytest.mark.parametrize("layout,group,n,k,m,x_type", [
@@ -106,9 +131,10 @@ def test_odd_stages_across_tiles(qx, orc, oracle_mod, layout, group, n, k, m, x_
     assert qx.lib.qx_check_device_errors() == qx.OK, qx.last_error()
 
 
-def test_act_order_and_unaligned_activations(qx, orc, oracle_mod):
+@pytest.mark.parametrize("n", [900, 1100])  # the digit kernels, the tensor cores
+def test_act_order_and_unaligned_activations(qx, orc, oracle_mod, n):
     import torch
-    n, k, m = 900, 1024, 40
+    k, m = 1024, 40
     rng = np.random.Generator(np.random.Philox(key=[5, 6]))
     order = rng.permutation(k).astype(np.int32)
     weights, tensor = _tensor(qx, oracle_mod, rng, INT4, 128, n, k, act_order=order)
@@ -127,8 +153,8 @@ def test_act_order_and_unaligned_activations(qx, orc, oracle_mod):
     assert close(out.cpu().numpy(), orc.canonical_gemm_f64(plain_tensor, np.ascontiguousarray(x_exact), F32, m))
 
 
-def test_a_token_that_is_not_finite_stays_alone(qx, orc, oracle_mod):
-    n, k, m = 2048, 1024, 33
+@pytest.mark.parametrize("n,k,m", [(2048, 1024, 33), (4096, 1024, 40)])  # (f32: digit kernels, tensor cores)
+def test_a_token_that_is_not_finite_stays_alone(qx, orc, oracle_mod, n, k, m):
     rng = np.random.Generator(np.random.Philox(key=[8, 9]))
     weights, tensor = _tensor(qx, oracle_mod, rng, UINT4, 64, n, k)
     x = (rng.standard_normal((m, k)) * 0.1).astype(np.float32)

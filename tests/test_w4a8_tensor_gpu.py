@@ -11,6 +11,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("m,n,k", [
     (2, 128, 258),      # smallest batch and matrix of rows that start on any byte
     (13, 128, 256),     # ... and of rows on whole vectors
+    (4, 128, 258),      # the smallest of both above the lines of the small matrices
+    (17, 128, 256),
     (1, 4096, 2050),    # one row of a large matrix
     (33, 129, 1033),    # an odd number of columns; a second tile of one row
     (64, 300, 2050),
