@@ -393,7 +393,8 @@ QX_API const char* qx_lowbit_gemm_variant(int format);
  * per row), the dot is an exact integer, Y = float(dot) * weight_scale[o] * activation_scale[r]
  * -- bit-identical to the reference. HOST pointers; the _dev form takes device pointers plus
  * qx_lowbit_w8a8_scratch_bytes(m, k) bytes of device scratch (it allocates nothing). The size
- * never falls as m or k grows: a scratch for the largest call serves every smaller one. */
+ * never falls as m or k grows: a scratch for the largest call serves every smaller one. Nothing is
+ * read before the work in front of the call on its stream has finished, the weights included. */
 QX_API qx_status qx_lowbit_gemm_w8a8(const uint8_t* packed_weights, const float* weight_scales,
                               const float* x, float* y, long long m, long long n, long long k);
 QX_API size_t qx_lowbit_w8a8_scratch_bytes(long long m, long long k);

@@ -382,14 +382,22 @@ __global__ void __launch_bounds__(32 * WARPS) canonical_gemm_kernel(const Canoni
 // 32 envelopes, then 32 span sums.
 constexpr int kImageWords = 3 * 128 + 32 + 32;
 
+// Internal fourth layout of the digit kernels: adjacent nibbles meaning nibble - 8 (the compact
+// int4 rows of lowbit_gemm, kernels/quantization/lowbit_ref.cpp:229-256): the symmetric path
+// without the xor.
+constexpr int kLayoutInt4Offset8 = 3;
+
 template <int LAYOUT>
 __global__ void __launch_bounds__(128) canonical_digits_prepass(const CanonicalParams p,
                                                                 uint32_t* __restrict__ image) {
   // Let the projection kernel behind start (it fetches weights first), then wait for the
   // work in front: the activations may be its output, and the projection of the previous
-  // call may still be reading the images this kernel overwrites.
-  asm volatile("griddepcontrol.launch_dependents;");
+  // call may still be reading the images this kernel overwrites. Compact int4 rows are the
+  // caller's, not a prepared tensor's, so that work in front may have written them as well:
+  // there the projection kernel starts behind the wait.
+  if (LAYOUT != kLayoutInt4Offset8) asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (LAYOUT == kLayoutInt4Offset8) asm volatile("griddepcontrol.launch_dependents;");
   constexpr bool kInt8 = LAYOUT == QX_CANONICAL_INT8_SYMMETRIC;
   const int columns = static_cast<int>(p.columns);
   const int chunks = (columns + kChunk - 1) / kChunk;
@@ -488,7 +496,7 @@ __device__ __forceinline__ float span_dot(const uint32_t (&w)[4], const uint4& d
   s0 = dp4a_us(w[3], d0.w, s0); s1 = dp4a_us(w[3], d1.w, s1); s2 = dp4a_us(w[3], d2.w, s2);
   // sum(u * t): |.| <= 16 * 15 * 2^22 < 2^30, exact in int32
   const int ut = (s2 << 16) + (s1 << 8) + s0;
-  if (LAYOUT == QX_CANONICAL_INT4_SYMMETRIC || LAYOUT == 3 /* kLayoutInt4Offset8 */) {
+  if (LAYOUT == QX_CANONICAL_INT4_SYMMETRIC || LAYOUT == kLayoutInt4Offset8) {
     return __int2float_rn(ut - 8 * tsum);  // u = code + 8
   }
   // affine: sum((u - zero) * t) = sum(u * t) - zero * sum(t); exact in int32 when the tensor's
@@ -496,11 +504,6 @@ __device__ __forceinline__ float span_dot(const uint32_t (&w)[4], const uint4& d
   if (integral_zero) return __int2float_rn(ut - __float2int_rn(zero) * tsum);
   return fmaf(-zero, __int2float_rn(tsum), __int2float_rn(ut));
 }
-
-// Internal fourth layout of the digit kernels: adjacent nibbles meaning nibble - 8 (the compact
-// int4 rows of lowbit_gemm, kernels/quantization/lowbit_ref.cpp:229-256): the symmetric path
-// without the xor.
-constexpr int kLayoutInt4Offset8 = 3;
 
 constexpr int kDigitWarps = 4;  // independent warps per CTA: no shared memory, no barrier
 constexpr int kStep = 1;       // chunks a lane requests at once (measured: 1 is as fast as 4)

@@ -85,15 +85,17 @@ __global__ void __launch_bounds__(256) quantize_int8_kernel(const float* __restr
 // Long groups (a whole activation row of a few thousand elements): one block per group, so
 // the row is read with 256 lanes instead of 32. Same values: max and the integer sum do not
 // depend on the order. It lets the kernel behind it (the W4A8 GEMM, which first fetches
-// weights) start at once and waits for the kernel in front itself.
+// weights) start as soon as the kernel in front is done.
 __global__ void __launch_bounds__(256) quantize_int8_block_kernel(const float* __restrict__ x,
                                                                   int8_t* __restrict__ codes,
                                                                   float* __restrict__ scales,
                                                                   int* __restrict__ code_sums,
                                                                   long long group_size) {
-  asm volatile("griddepcontrol.launch_dependents;");
   // x may be the output of the kernel in front, and the codes are read by the GEMM in front
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  // (behind the wait: the GEMM fetches weights, which are the caller's, before it waits itself, and
+  // the kernel in front may have written them)
+  asm volatile("griddepcontrol.launch_dependents;");
   __shared__ float warp_max[8];
   __shared__ int warp_sum[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -136,9 +138,11 @@ __global__ void __launch_bounds__(256) quantize_codes_f16_kernel(const float* __
                                                                  float* __restrict__ scales,
                                                                  int* __restrict__ counters, int counter_count,
                                                                  long long k, long long stride) {
-  asm volatile("griddepcontrol.launch_dependents;");
   // x may be the output of the kernel in front, and the codes are read by the GEMM in front
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  // (behind the wait: the GEMM fetches weights, which are the caller's, before it waits itself, and
+  // the kernel in front may have written them)
+  asm volatile("griddepcontrol.launch_dependents;");
   __shared__ float warp_max[8];
   const long long row = blockIdx.x;
   const float* in = x + row * k;

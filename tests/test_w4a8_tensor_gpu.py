@@ -111,3 +111,27 @@ def test_scratch_of_the_largest_call_serves_smaller_ones(qx, orc):
         torch.cuda.synchronize()
         assert np.array_equal(y.cpu().numpy().view(np.uint32), _exact(orc, packed, scales, x, m, n, k).view(np.uint32))
         assert bool((scratch[size:] == 0xA5).all())
+
+
+# Weights written by the kernel directly in front, other ones on every call: nothing of them may be
+# fetched before that kernel is done (dp4a kernel, tensor cores with rows on vectors and on any byte)
+@pytest.mark.parametrize("m,n,k", [(1, 14336, 4096), (8, 4096, 4096), (32, 8192, 4096), (16, 8192, 4098)])
+def test_weights_written_in_front(qx, orc, m, n, k):
+    import torch
+    rng = np.random.Generator(np.random.Philox(key=[m, n, k][:2]))
+    sides = [torch.from_numpy(rng.integers(0, 256, (n, k // 2), dtype=np.uint8)).cuda() for _ in range(2)]
+    scales = rng.uniform(0.001, 0.1, n).astype(np.float32)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    want = [torch.from_numpy(_exact(orc, side.cpu().numpy(), scales, x, m, n, k)).cuda() for side in sides]
+    scratch = torch.zeros(int(qx.lib.qx_lowbit_w8a8_scratch_bytes(m, k)), dtype=torch.uint8, device="cuda")
+    w, ws, xd = torch.zeros_like(sides[0]), torch.from_numpy(scales).cuda(), torch.from_numpy(x).cuda()
+    outputs = [torch.full((m, n), np.nan, device="cuda") for _ in range(20)]
+    torch.cuda.synchronize()
+    for i, y in enumerate(outputs):
+        torch.bitwise_xor(sides[i % 2], 0, out=w)
+        status = qx.lib.qx_lowbit_gemm_w8a8_dev(w.data_ptr(), ws.data_ptr(), xd.data_ptr(), y.data_ptr(),
+                                                scratch.data_ptr(), m, n, k, torch.cuda.current_stream().cuda_stream)
+        assert status == qx.OK, qx.last_error()
+    torch.cuda.synchronize()
+    for i, y in enumerate(outputs):
+        assert torch.equal(y, want[i % 2]), i
