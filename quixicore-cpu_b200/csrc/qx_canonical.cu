@@ -76,6 +76,7 @@ struct qx_canonical_weights {
   int* group_index = nullptr;   // device: [columns] packed column -> scale group, or null
   int* act_order = nullptr;     // device: [columns] packed column -> activation column, or null
   bool integral_zeros = false;  // every zero point is one of 0, 1, .. 15 (the usual case)
+  bool scales_have_room = true;  // every scale times 2^16 is finite (qx_tile_pipe.cuh)
 };
 
 namespace qx {
@@ -1016,7 +1017,7 @@ qx_status launch_any(const CanonicalParams& p, bool digits, uint32_t* image, int
 // (512 f16 tokens, 4096 x 4096: 1.5e-7 against 4.5e-8 of the result).
 bool scaled_route(const qx_canonical_weights* w, int x_type, long long m) {
   // a tile is 128 weight rows: smaller matrices would be mostly padding
-  if (w->group_index != nullptr || w->rows < 128) return false;
+  if (w->group_index != nullptr || w->rows < 128 || !w->scales_have_room) return false;
   // fractional zero points have no exact 16-bit form
   if (w->layout == QX_CANONICAL_UINT4_AFFINE && !w->integral_zeros) return false;
   if (w->layout == QX_CANONICAL_INT8_SYMMETRIC && w->groups_per_row == 1) return false;
@@ -1349,6 +1350,9 @@ qx_status qx_canonical_prepare(const qx_canonical_tensor* tensor, qx_canonical_w
       w->integral_zeros = false;
       break;
     }
+  }
+  for (size_t i = 0; i < tensor->scale_count; ++i) {
+    if (tensor->scales[i] >= 0x1p111f) w->scales_have_room = false;
   }
   // one allocation: codes, then every table on a 256-byte boundary
   const size_t scale_offset = align_up(tensor->data_bytes, 256);

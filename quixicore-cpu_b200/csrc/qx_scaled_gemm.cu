@@ -9,7 +9,9 @@
 // three bf16 planes whose sum is the value, multiplied one after the other into the same
 // accumulator). So every product is exact, a group's sum is formed by the tensor core in f32
 // over at most 128 columns, and the f32 scale is applied once per group by an f32 multiply-add
-// on the CUDA cores: no scale is ever rounded to 16 bits.
+// on the CUDA cores: no scale is ever rounded to 16 bits. Whole numbers in bf16 carry 2^-16, so
+// that no group's sum leaves the range of f32. (f32 tokens that are below 2^-110 altogether lose
+// low bits: their third plane is below the smallest bf16.)
 //
 // Pipeline (persistent CTAs, one per SM, 28 warps):
 //   warp 0       packed codes: 16 KiB slots of [128 rows][128 bytes], 128-byte swizzled
@@ -167,11 +169,11 @@ struct Walk {
 };
 
 // Eight nibbles -> eight 16-bit whole numbers nibble - z in column order. A nibble under the
-// exponent bits of `magic` (f16 1024 = 0x6400, bf16 128 = 0x4300: unit steps) is base + nibble;
+// exponent bits of `magic` (f16 1024 = 0x6400, bf16 128 times 2^-16: steps of one) is base + nibble;
 // `base_z` holds base + z twice.
 template <bool BF16>
 __device__ __forceinline__ uint4 convert_nibbles(uint32_t w, uint32_t base_z) {
-  const uint32_t magic = BF16 ? 0x43004300u : 0x64006400u;
+  const uint32_t magic = BF16 ? kBf16Base * 0x10001u : 0x64006400u;
   const uint32_t high = w >> 4;
   uint32_t out[4];
 #pragma unroll
@@ -186,7 +188,7 @@ template <bool BF16>
 __device__ __forceinline__ uint32_t zero_word(float z) {
   uint32_t bits;
   if (BF16) {
-    bits = __float_as_uint(128.0f + z) >> 16;  // exact: 128 .. 143
+    bits = __float_as_uint((128.0f + z) / kBf16Unscale) >> 16;  // exact: 128 .. 143
   } else {
     bits = __half_as_ushort(__float2half_rn(1024.0f + z));
   }
@@ -448,6 +450,7 @@ scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       // 16 columns at a time: with 32 of them in registers the loop spills (q8_0, 331 tokens on
       // 4096 x 11008: 147 us against 139).
       auto add_unit = [&](uint32_t taddr, float scale, bool release) {
+        if (BF16) scale *= kBf16Unscale;
         const unsigned long long s2 = pack2(__float_as_uint(scale), __float_as_uint(scale));
 #pragma unroll
         for (int c = 0; c < S::kCols; c += 16) {

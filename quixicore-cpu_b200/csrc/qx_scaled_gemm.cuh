@@ -16,7 +16,7 @@ enum ScaledGemmSource {
 struct ScaledGemmArgs {
   ScaledGemmSource source;
   const uint8_t* codes;      // device: codes or panel
-  const float* scales;       // [rows][columns / group] (not for the panel)
+  const float* scales;       // [rows][columns / group] below 2^111 (not for the panel)
   const float* zeros;        // nibbles: zero point beside every scale, whole numbers 0 .. 15;
                              // null: 8 everywhere
   uint32_t nibble_xor;       // 0x88888888 for two's complement nibbles, else 0

@@ -64,6 +64,12 @@ __device__ __forceinline__ void add_with_rest2(unsigned long long& total, unsign
 }
 
 // ---- 16-bit whole numbers ----------------------------------------------------------------
+// bf16 ones carry 2^-16: a group's sum of bf16 activations of any size then stays finite in f32
+// (2^128 * 2^8 * 128 columns * 2^-16), and no bit of a normal activation's product falls below
+// 2^-149. The scales carry 2^16 in return. f16 activations are small enough as they are.
+constexpr float kBf16Unscale = 65536.0f;
+constexpr uint32_t kBf16Base = 0x3B00u;  // 128 * 2^-16: unit steps of 2^-16
+
 template <bool BF16>
 __device__ __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) {
   if (BF16) {
@@ -74,29 +80,18 @@ __device__ __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) {
   const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
   return *reinterpret_cast<const uint32_t*>(&v);
 }
-// Two signed bytes of `w` picked by `selector` -> two 16-bit whole numbers.
+// Two signed bytes of `w` picked by `selector` (its upper bytes take byte 4) -> two 16-bit whole
+// numbers.
 template <bool BF16>
 __device__ __forceinline__ uint32_t convert_bytes2(uint32_t w, uint32_t selector) {
   if (BF16) {
-    // (128 + low seven bits) - (128, or 256 for a negative code)
-    const uint32_t p = __byte_perm(w, 0x43434343u, selector);
+    // (128 + low seven bits) - (128, or 256 for a negative code), all times 2^-16
+    const uint32_t p = __byte_perm(w, kBf16Base >> 8, selector);
     return sub2<true>(p & 0xFF7FFF7Fu, p & 0xFF80FF80u);
   }
   // code ^ 0x80 = code + 128 under the exponent of 1024
   const uint32_t p = __byte_perm(w ^ 0x80808080u, 0x64646464u, selector);
   return sub2<false>(p, 0x64806480u);
-}
-
-// ---- TMEM -------------------------------------------------------------------------------
-// 16 columns into the first half of `r`
-__device__ __forceinline__ void tmem_ld_32x16_low(uint32_t taddr, uint32_t (&r)[32]) {
-  uint32_t low[16];
-  sm100::tmem_ld_32x16(taddr, low);
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    r[i] = low[i];
-    r[16 + i] = 0u;
-  }
 }
 
 }  // namespace tile

@@ -169,6 +169,65 @@ def test_a_token_that_is_not_finite_stays_alone(qx, orc, oracle_mod, n, k, m):
         assert close(y[finite], exact)
 
 
+# Activations near the ends of their type's range: a group's sum of whole weights times activations
+# is far beyond f32 where the scaled result is not, and down to the smallest normal numbers
+@pytest.mark.parametrize("layout,group,n,k,m,x_type,size", [
+    (UINT4, 128, 1100, 1024, 64, BF16, 1e37), (UINT4, 128, 1100, 1024, 64, BF16, 1e-36),
+    (INT8, 128, 2048, 1024, 100, BF16, 1e36), (INT8, 128, 2048, 1024, 100, BF16, 1e-36),
+    (INT4, 32, 4096, 1024, 40, F32, 2e37), (INT4, 32, 4096, 1024, 40, F32, 1e-28)])
+def test_activations_of_extreme_size(qx, oracle_mod, layout, group, n, k, m, x_type, size):
+    rng = np.random.Generator(np.random.Philox(key=[n + k, m + group]))
+    weights, tensor = _tensor(qx, oracle_mod, rng, layout, group, n, k)
+    x, x_exact = _storage((rng.standard_normal((m, k)) * size).astype(np.float32), x_type)
+    exact = _product_f64(tensor, x_exact)
+    status, y = weights.qgemm_storage(x, x_type, m)
+    assert status == qx.OK, qx.last_error()
+    assert np.all(np.isfinite(y))
+    # (1e-5: far above f32 sums, far below one overflow or a lost plane)
+    assert np.linalg.norm((y - exact) / size) <= 1e-5 * np.linalg.norm(exact / size)
+
+
+@pytest.mark.parametrize("size", [1e36, 1e-30])
+def test_q8_0_prefill_of_extreme_size(qx, orc, wl, size):
+    import torch
+    n, k, m = 512, 1024, 40
+    packed = wl.packed_blocks(0, n, k, 0.001, 0.02, seed=9)
+    xb = wl.to_bf16_bits(wl.activations_f32(m, k, seed=m) * np.float32(size))
+    weights = qx.PackedWeights()
+    assert weights.prepare(0, packed, n, k) == qx.OK, qx.last_error()
+    y = torch.zeros((m, n), device="cuda")
+    assert weights.qgemm_bf16_dev(torch.from_numpy(xb.view(np.int16)).cuda(), y, m) == qx.OK, qx.last_error()
+    torch.cuda.synchronize()
+    _, exact = orc.qgemm_f64(0, packed, wl.bf16_bits_to_f32(xb), m, n, k)
+    got = y.cpu().numpy().astype(np.float64)
+    assert np.all(np.isfinite(got))
+    assert np.linalg.norm((got - exact) / size) <= 1e-5 * np.linalg.norm(exact / size)
+
+
+@pytest.mark.parametrize("x_type", [F32, F16, BF16])
+def test_an_infinite_activation(qx, oracle_mod, x_type):
+    """16-bit types: an infinity of the weight's sign, or NaN where the weight is zero, as the reference's
+    sums give; f32: NaN in the whole token. Other tokens do not see it."""
+    n, k, m = 4096, 1024, 40
+    rng = np.random.Generator(np.random.Philox(key=[18, 19]))
+    weights, tensor = _tensor(qx, oracle_mod, rng, UINT4, 64, n, k)
+    x = (rng.standard_normal((m, k)) * 0.1).astype(np.float32)
+    x[7, 100] = np.inf
+    stored, values = _storage(x, x_type)
+    status, y = weights.qgemm_storage(stored, x_type, m)
+    assert status == qx.OK, qx.last_error()
+    finite = [r for r in range(m) if r != 7]
+    assert close(y[finite], _product_f64(tensor, values[finite]))
+    if x_type == F32:
+        assert np.all(np.isnan(y[7]))
+    else:
+        column = np.zeros((1, k), np.float32)
+        column[0, 100] = 1.0
+        weight = _product_f64(tensor, column)[0]
+        assert np.array_equal(y[7] == np.inf, weight > 0) and np.array_equal(y[7] == -np.inf, weight < 0)
+        assert np.array_equal(np.isnan(y[7]), weight == 0)
+
+
 @pytest.mark.parametrize("n,k,m", [(128, 256, 16), (300, 1056, 33), (257, 416, 64), (640, 2080, 65), (384, 11008, 331)])
 def test_q8_0_prefill(qx, orc, wl, n, k, m):
     import torch
