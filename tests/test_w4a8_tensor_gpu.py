@@ -18,24 +18,46 @@ pytestmark = pytest.mark.gpu
     (64, 300, 2050),
     (65, 257, 1502),    # first large tile
     (130, 200, 1312),   # whole tiles only
-    (5, 128, 16510),    # sums up to the largest that stay below 2^24
-    (5, 128, 16514),    # one step further: the integer kernel
+    (5, 128, 16510),    # the longest rows of the tensor cores, and one step further: the integer kernel
+    (5, 128, 16514),    # (sums up to the limit: test_sums_at_the_limit)
 ])
 def test_bits_of_the_reference(qx, orc, m, n, k):
     rng = np.random.Generator(np.random.Philox(key=[m * 1000 + n, k]))
     packed = rng.integers(0, 256, (n, (k + 1) // 2), dtype=np.uint8)
-    if k >= 16000:  # the largest sums: every product is -8 * 127 or 8 * 127
-        packed[:] = 0
     scales = rng.uniform(0.001, 0.1, n).astype(np.float32)
     x = rng.standard_normal((m, k)).astype(np.float32)
-    if k >= 16000:
-        x = np.ones_like(x)
     x[m // 2, ::5] = 0.0
     status, y = qx.lowbit_gemm_w8a8(packed.reshape(-1), scales, x, m, n, k)
     assert status == qx.OK, qx.last_error()
     _, want = orc.lowbit_gemm_w8a8(packed.reshape(-1), scales, x, m, n, k)
     assert np.array_equal(np.asarray(y).view(np.uint32).reshape(m, n), np.asarray(want).view(np.uint32).reshape(m, n))
     assert qx.lib.qx_check_device_errors() == qx.OK, qx.last_error()
+
+
+@pytest.mark.parametrize("k", [16510, 16512, 20001])
+def test_sums_at_the_limit(qx, orc, k):
+    """Products of -8 * 127 behind a few of 1 * 127: odd sums just below 2^24, which lose their last bit as
+    soon as f32 or the tensor core rounds anything, and sums beyond it for the integer kernel."""
+    m, n = 20, 130
+    column, row = np.arange(k + k % 2)[None, :], np.arange(n)[:, None]
+    nibbles = np.where(column < 2 * (row % 8) + 1, 9, 0).astype(np.uint8)  # odd numbers of early columns
+    if k > 16512:
+        nibbles[(column >= 256) & (column % 128 == 7) & (column % (256 + 128 * (row % 5)) < 128)] = 9
+    packed = np.ascontiguousarray(nibbles[:, 0::2] | (nibbles[:, 1::2] << 4))
+    scales = np.full(n, 0.5, np.float32)
+    x = np.ones((m, k), np.float32)
+    dots = 127 * (nibbles[:, :k].astype(np.int64) - 8).sum(axis=1)
+    parts = np.add.reduceat((nibbles[:, :k].astype(np.int64) - 8) * 127, np.arange(0, k, 128), axis=1)
+    chain = np.add.accumulate(parts.astype(np.float32), axis=1, dtype=np.float32)[:, -1]
+    if k <= 16512:
+        assert np.all((np.abs(dots) > 1 << 23) & (np.abs(dots) < 1 << 24) & (dots % 2 == 1))
+    else:  # f32 sums of 128 columns would end elsewhere
+        assert np.any(chain != dots.astype(np.float32))
+    status, y = qx.lowbit_gemm_w8a8(packed.reshape(-1), scales, x, m, n, k)
+    assert status == qx.OK, qx.last_error()
+    _, want = orc.lowbit_gemm_w8a8(packed.reshape(-1), scales, x, m, n, k)
+    assert np.array_equal(want[0], dots.astype(np.float32) * np.float32(0.5) * (np.float32(1.0) / np.float32(127.0)))
+    assert np.array_equal(np.asarray(y).view(np.uint32).reshape(m, n), np.asarray(want).view(np.uint32).reshape(m, n))
 
 
 def _exact(orc, packed, scales, x, m, n, k):
