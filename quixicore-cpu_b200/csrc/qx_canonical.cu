@@ -1077,6 +1077,19 @@ qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_t
   // float multiply-adds on weights decoded one by one
   const bool digits = w->group_index == nullptr &&
                       (p.groups_per_row == 1 || p.group_size % kElems == 0);
+  // workspace behind its counters: [gathered activations (act-order)][digit images]
+  const size_t gather_bytes =
+      w->act_order != nullptr ? align_up(static_cast<size_t>(m) * w->columns * sizeof(float), 256) : 0;
+  // int8 with one scale per row, five tokens or more: the tensor-core route
+  long long prefill_from = kPrefillTokens;
+  // developer switch: QX_B200_CANONICAL_PREFILL_TOKENS=<n> moves the threshold
+  if (const char* forced = std::getenv("QX_B200_CANONICAL_PREFILL_TOKENS")) {
+    const long long asked = std::atoll(forced);
+    if (asked > 0) prefill_from = asked;
+  }
+  const bool prefill = int8 && p.groups_per_row == 1 && m >= prefill_from && w->columns <= 131000;
+  const size_t image_bytes = prefill ? prefill_scratch_bytes(m, w->rows, w->columns)
+                                     : (digits ? digit_image_bytes(m, w->columns) : 0);
   // batches on the tensor cores with the scales applied per group (qx_scaled_gemm.cu)
   ScaledGemmArgs scaled{};
   scaled.source = int8 ? kScaledBytes : kScaledNibbles;
@@ -1098,24 +1111,15 @@ qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_t
   scaled.ldy = w->rows;
   if (scaled_route(w, x_type, m) && scaled_gemm_serves(scaled)) {
     const int sm_count = ctx->prop.multiProcessorCount;
-    QX_TRY(workspace->reserve(kWorkspaceCounterBytes + scaled_gemm_scratch_bytes(scaled, sm_count)));
+    // (and what the digit kernels of smaller batches use)
+    const size_t scaled_bytes = scaled_gemm_scratch_bytes(scaled, sm_count);
+    QX_TRY(workspace->reserve(kWorkspaceCounterBytes + (scaled_bytes > gather_bytes + image_bytes
+                                                            ? scaled_bytes
+                                                            : gather_bytes + image_bytes)));
     return launch_scaled_gemm(scaled, static_cast<uint8_t*>(workspace->base) + kWorkspaceCounterBytes,
                               static_cast<int*>(workspace->base), kWorkspaceCounterBytes, sm_count,
                               ctx->error_dev, stream);
   }
-  // workspace behind its counters: [gathered activations (act-order)][digit images]
-  const size_t gather_bytes =
-      w->act_order != nullptr ? align_up(static_cast<size_t>(m) * w->columns * sizeof(float), 256) : 0;
-  // int8 with one scale per row, five tokens or more: the tensor-core route
-  long long prefill_from = kPrefillTokens;
-  // developer switch: QX_B200_CANONICAL_PREFILL_TOKENS=<n> moves the threshold
-  if (const char* forced = std::getenv("QX_B200_CANONICAL_PREFILL_TOKENS")) {
-    const long long asked = std::atoll(forced);
-    if (asked > 0) prefill_from = asked;
-  }
-  const bool prefill = int8 && p.groups_per_row == 1 && m >= prefill_from && w->columns <= 131000;
-  const size_t image_bytes = prefill ? prefill_scratch_bytes(m, w->rows, w->columns)
-                                     : (digits ? digit_image_bytes(m, w->columns) : 0);
   uint32_t* image = nullptr;
   if (gather_bytes + image_bytes != 0) {
     QX_TRY(workspace->reserve(kWorkspaceCounterBytes + gather_bytes + image_bytes));

@@ -465,6 +465,14 @@ qx_status launch_q4_gemm_bf16(const qx_weights* w, const uint16_t* x_bf16_dev, f
       m * w->columns < (1LL << 40)) {
     return launch_tc(w, x_bf16_dev, y_dev, m, ldy, ws, stream);
   }
+  const long long count = m * w->columns;
+  DeviceContext* ctx = nullptr;
+  QX_TRY(current_context(&ctx));
+  GemvScratch scratch;
+  QX_TRY(gemv_scratch_layout(w, static_cast<int>(m < kGemvMaxBatch ? m : kGemvMaxBatch),
+                             ctx->prop.multiProcessorCount, &scratch));
+  const size_t table_bytes = align_up(scratch.total_bytes, 256);
+  const size_t exact_bytes = table_bytes + static_cast<size_t>(count) * sizeof(float);
   if (w->format == QX_FORMAT_Q8_0 && w->segments == 1 && scaled_prefill(w, m)) {
     ScaledGemmArgs a{};
     a.source = kScaledPanelQ8;
@@ -480,10 +488,10 @@ qx_status launch_q4_gemm_bf16(const qx_weights* w, const uint16_t* x_bf16_dev, f
     a.y_type = QX_STORAGE_F32;
     a.ldy = ldy;
     if (scaled_gemm_serves(a)) {
-      DeviceContext* ctx = nullptr;
-      QX_TRY(current_context(&ctx));
       const int sm_count = ctx->prop.multiProcessorCount;
-      QX_TRY(ws->reserve(kWorkspaceCounterBytes + scaled_gemm_scratch_bytes(a, sm_count)));
+      const size_t scaled_bytes = kWorkspaceCounterBytes + scaled_gemm_scratch_bytes(a, sm_count);
+      // (and what the exact path of smaller batches uses)
+      QX_TRY(ws->reserve(scaled_bytes > exact_bytes ? scaled_bytes : exact_bytes));
       return launch_scaled_gemm(a, static_cast<uint8_t*>(ws->base) + kWorkspaceCounterBytes,
                                 static_cast<int*>(ws->base), kWorkspaceCounterBytes, sm_count,
                                 ctx->error_dev, stream);
@@ -492,14 +500,7 @@ qx_status launch_q4_gemm_bf16(const qx_weights* w, const uint16_t* x_bf16_dev, f
   // Exact path: widen the activations to f32 (bf16 -> f32 is exact) and reuse the f32
   // batched kernel; its scratch sits at the start of the workspace and the widened copy
   // behind it.
-  const long long count = m * w->columns;
-  DeviceContext* ctx = nullptr;
-  QX_TRY(current_context(&ctx));
-  GemvScratch scratch;
-  QX_TRY(gemv_scratch_layout(w, static_cast<int>(m < kGemvMaxBatch ? m : kGemvMaxBatch),
-                             ctx->prop.multiProcessorCount, &scratch));
-  const size_t table_bytes = align_up(scratch.total_bytes, 256);
-  QX_TRY(ws->reserve(table_bytes + static_cast<size_t>(count) * sizeof(float)));
+  QX_TRY(ws->reserve(exact_bytes));
   float* x_f32 = reinterpret_cast<float*>(static_cast<uint8_t*>(ws->base) + table_bytes);
   const unsigned grid = static_cast<unsigned>(min((count + 255) / 256, 4096LL));
   bf16_to_f32_kernel<<<grid, 256, 0, stream>>>(x_bf16_dev, x_f32, count);

@@ -816,7 +816,7 @@ __global__ void __launch_bounds__(256) stage_activations_kernel(const void* __re
 struct Plan {
   bool small, staged, split;
   int bn, planes, promote, slabs, columns, o_tiles, r_tiles, grid;
-  size_t staged_bytes, partial_bytes;
+  size_t staged_bytes;
 };
 
 Plan make_plan(const ScaledGemmArgs& a, int sm_count) {
@@ -851,7 +851,6 @@ Plan make_plan(const ScaledGemmArgs& a, int sm_count) {
   p.split = !a.whole_tiles && even < whole && units < (1LL << 30);
   const long long pieces = p.split ? units : tiles;
   p.grid = static_cast<int>(pieces < sm_count ? pieces : sm_count);
-  p.partial_bytes = p.split ? static_cast<size_t>(p.grid) * 2 * kRows * p.bn * sizeof(float) : 0;
   return p;
 }
 
@@ -931,8 +930,10 @@ bool scaled_gemm_serves(const ScaledGemmArgs& a) {
 }
 
 size_t scaled_gemm_scratch_bytes(const ScaledGemmArgs& a, int sm_count) {
-  const Plan plan = make_plan(a, sm_count);
-  return plan.staged_bytes + plan.partial_bytes;
+  const int planes = a.source == kScaledPanelQ8 ? 1 : 3;
+  const size_t tokens = a.m <= 32 ? 32 : (a.m <= 64 ? 64 : Large::kTokens);
+  return align_up(static_cast<size_t>(planes) * a.m * a.columns * 2, 256) +
+         static_cast<size_t>(sm_count) * 2 * kRows * tokens * sizeof(float);
 }
 
 qx_status launch_scaled_gemm(const ScaledGemmArgs& a, void* scratch, int* counters, size_t counter_bytes,

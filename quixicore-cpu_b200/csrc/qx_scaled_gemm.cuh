@@ -41,7 +41,9 @@ struct ScaledGemmArgs {
 // Whether the sizes and pointers are ones that the kernel takes (not whether it is the better
 // choice: that is the caller's rule).
 bool scaled_gemm_serves(const ScaledGemmArgs& a);
-// Scratch behind the workspace's counters that launch_scaled_gemm() uses.
+// Scratch behind the workspace's counters for launch_scaled_gemm(): enough for `a` and for every
+// call of fewer tokens, of any type and alignment, on the same tensor, so that a workspace which
+// has served the largest batch does not grow any more (it could not under stream capture).
 size_t scaled_gemm_scratch_bytes(const ScaledGemmArgs& a, int sm_count);
 // Bytes of counters that a launch of at most `ctas` CTAs uses: a CTA holds the first piece of at
 // most two tiles, and every epilogue warp counts for itself.
