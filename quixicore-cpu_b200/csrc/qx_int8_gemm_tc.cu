@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(kThreads, 1) int8_gemm_tc_kernel(
     const int quarter = warp & 3;
     const int half = (warp - 2) >> 2;
     const int epi_thread = threadIdx.x - 64;  // 0..255
-    uint32_t acc = 0, acc_phase = 0;
+    uint32_t acc = 0, acc_phase = 0, table = 0;
     bool ok = true;
     int* last_flag = zp_tile + 2 * 256;  // one word behind the staged tables
     // Scales one 32-token chunk of exact accumulators v[] (channel o, tokens rc..rc+31)
@@ -356,9 +356,13 @@ __global__ void __launch_bounds__(kThreads, 1) int8_gemm_tc_kernel(
       const bool whole = seg.ks0 == 0 && seg.ks1 == p.k_slabs;
       const long long o_base = static_cast<long long>(tile / p.r_tiles) * (NA * kBM) + quarter * 32 + lane;
       const long long r0 = static_cast<long long>(tile % p.r_tiles) * p.bn;
-      // stage this tile's activation scales (and zero points) for broadcast reads
-      float* as_s = as_tile + acc * 256;
-      int* zp_s = zp_tile + acc * 256;
+      // Stage this tile's activation scales (and zero points) for broadcast reads, into the halves
+      // of the tables by turns whatever the number of accumulators: a warp that is done with a
+      // tile gets here while others still read that tile's, and the barrier below says that all of
+      // them are done with the one before.
+      float* as_s = as_tile + table * 256;
+      int* zp_s = zp_tile + table * 256;
+      table ^= 1u;
       for (int i = epi_thread; i < p.bn; i += 32 * kEpiWarps) {
         const long long r = r0 + i;
         as_s[i] = r < p.m ? p.as[r] : 0.0f;

@@ -128,3 +128,30 @@ def test_stream_k_split_is_exact(qx, orc, wl, shape, asym, monkeypatch):
     for mode, ys in results.items():
         for y in ys:
             assert_bit_equal(y, ref, f"stream_k={mode} {shape} asym={asym}")
+
+
+# More tiles of 256 channels than SMs, and tiles of other tokens behind a CTA's first one: every tile has
+# to be finished with its own tokens' scales, however far the epilogue warps are apart. Two calls in turn.
+@pytest.mark.parametrize("m,n,k,azp", [(1917, 8169, 1664, False), (1393, 8443, 1232, False), (1269, 10880, 768, False),
+                                       (712, 14336, 256, True)])
+def test_scales_of_a_ctas_next_tile(qx, m, n, k, azp):
+    import torch
+    sides = []
+    for seed in (1, 2):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        w = torch.randint(-127, 128, (n, k), generator=g, device="cuda", dtype=torch.int8)
+        x = torch.randint(-127, 128, (m, k), generator=g, device="cuda", dtype=torch.int8)
+        ws = torch.rand(n, generator=g, device="cuda") * 0.01 + 0.001
+        xs = torch.rand(m, generator=g, device="cuda") * 0.05 + 0.005
+        acc, extra = x.double() @ w.double().T, {}
+        if azp:
+            extra = dict(row_sum=w.sum(dim=1, dtype=torch.int32),
+                         zp=torch.randint(-20, 21, (m,), generator=g, device="cuda", dtype=torch.int32))
+            acc -= extra["zp"].double()[:, None] * extra["row_sum"].double()[None, :]
+        sides.append((w, x, ws, xs, torch.zeros((m, n), device="cuda"), extra, (acc.float() * ws[None, :]) * xs[:, None]))
+    for _ in range(15):
+        for w, x, ws, xs, y, extra, _ in sides * 2:
+            assert qx.int8_gemm_dev(w, x, ws, xs, y, m, n, k, **extra) == qx.OK, qx.last_error()
+        torch.cuda.synchronize()
+        for *_, y, extra, want in sides:
+            assert torch.equal(y, want)
