@@ -31,7 +31,8 @@
 //           qx_scaled_gemm.cu, chosen by scaled_route below.
 // Inputs stored as f16 / bf16 are widened exactly, the output is rounded once at the store.
 // On the first two paths a token's result does not depend on the batch it is computed in; a
-// batch that crosses five tokens changes route and with it the rounding (same tolerance).
+// batch that crosses a line of a tensor-core route changes route and with it the rounding (same
+// tolerance).
 //
 // HBM layout. Codes stay in the canonical row-major byte order (a row of K int8 codes or
 // K/2 nibble pairs is already what a warp wants to stream with 16-byte loads), followed by

@@ -732,7 +732,7 @@ qx_status qx_lowbit_gemm_w8a8(const uint8_t* packed_weights, const float* weight
   return QX_STATUS_OK;
 }
 
-const char* qx_lowbit_gemm_w8a8_variant(void) { return "sm100a_dp4a_stream"; }
+const char* qx_lowbit_gemm_w8a8_variant(void) { return "sm100a_dp4a_stream+tcgen05_f16"; }
 
 const char* qx_lowbit_gemm_variant(int format) {
   return int4_format(format) ? "sm100a_digits_dp4a+stream_fma" : "unsupported";
