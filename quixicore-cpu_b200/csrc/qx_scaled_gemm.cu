@@ -631,6 +631,7 @@ scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
       }
     }
+    tmem_st_wait();  // (of totals, where the kernel gave up in the middle of a tile)
   } else {
     // -------------------------------- converters --------------------------------
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(S::kConvRegs));
