@@ -60,6 +60,7 @@
 #include "qx_gemv.cuh"
 #include "qx_int8_gemm.cuh"
 #include "qx_scaled_gemm.cuh"
+#include "qx_stream_mma.cuh"
 
 struct qx_canonical_weights {
   int layout = 0;
@@ -1037,6 +1038,32 @@ bool scaled_route(const qx_canonical_weights* w, int x_type, long long m) {
   return m >= (f32 ? 25 : 5) && m * w->rows * w->columns >= least;
 }
 
+// Which small batches stream the codes past their activations (qx_stream_mma.cu). Measured there | before (us):
+//   int8, one scale per row (four digit rows per token, exact sums): 14336 x 4096: 1 token 15.6 | 17.2, 4: 17.2 | 34.2,
+//     8: 20.6 | 20.7 (and one launch less);  4096 x 4096: 1: 6.0 | 6.8, 8: 8.2 | 12.6, 12: 9.9 | 15.2;  8192 x 4096:
+//     8: 10.9 | 17.0, 16: 21 | 17.7;  2048 x 4096: 16: 10.2 | 13.1
+//   16-bit tokens, scales along K (uint4, groups of 128): 14336 x 4096: 8 tokens 19.1 | 30.8, 16: 25.7 | 31.8, 32:
+//     36.2 | 32.0;  4096 x 4096: 32: 10.2 | 19.1;  8192 x 4096: 24: 19.5 | 23.3;  1024 x 8192, 16: 12.5 | 22.4;  groups
+//     of 32: 4096 x 4096, 8: 9.0 | 19.9, 8192 x 8192, 24: 68 | 55
+//   f32 tokens (three planes): 14336 x 4096: 16: 40 | 120;  4096 x 4096: 24: 18.4 | 58;  4096 x 11008: 8: 19 | 82
+// Not the smallest products, which are launches and nothing else on either route; and up to four tokens with scales
+// along K stay on the digit kernels, whose rows do not depend on the batch.
+constexpr long long kStreamWork = 1LL << 22;
+bool stream_digits_route(const qx_canonical_weights* w, long long m) {
+  return w->layout == QX_CANONICAL_INT8_SYMMETRIC && w->groups_per_row == 1 && m * w->rows * w->columns >= kStreamWork &&
+         (m <= 8 || (m <= kStreamColumns / 4 && m * w->rows <= (1LL << 16)));
+}
+bool stream_scaled_route(const qx_canonical_weights* w, int x_type, long long m) {
+  if (w->group_index != nullptr || !w->scales_have_room || m < 5 || m * w->rows * w->columns < kStreamWork) return false;
+  // fractional zero points have no exact 16-bit form; int8 with one scale per row has exact sums above
+  if (w->layout == QX_CANONICAL_UINT4_AFFINE && !w->integral_zeros) return false;
+  if (w->layout == QX_CANONICAL_INT8_SYMMETRIC && w->groups_per_row == 1) return false;
+  if (m > 16 && (m * w->rows > (1LL << 18) || (w->groups_per_row > 1 && w->group_size % 64 != 0))) return false;
+  return x_type != QX_STORAGE_F32 || m * w->rows * w->columns >= (1LL << 25);
+}
+// Their scratch: no more than a workspace has that served the calls before (it grows by whole MiB, counters in front).
+constexpr size_t kStreamScratchBytes = (1 << 20) - 4096;
+
 qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_type,
                            const float* bias, void* y, int y_type, long long m, int activation,
                            qx_workspace* workspace, cudaStream_t stream) {
@@ -1110,6 +1137,58 @@ qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_t
   scaled.y = y;
   scaled.y_type = y_type;
   scaled.ldy = w->rows;
+  if (stream_digits_route(w, m)) {
+    const size_t digit_bytes = align_up(stream_code_bytes(4 * m, w->columns), 256);
+    StreamIntArgs s{};
+    s.source = kStreamBytes;
+    s.result = kStreamDigits;
+    s.prepared = true;
+    s.codes = w->data;
+    s.x_rows = static_cast<int>(4 * m);
+    s.rows = w->rows;
+    s.columns = w->columns;
+    s.ws = w->scales;
+    s.bias = bias;
+    s.activation = activation;
+    s.y = y;
+    s.y_type = y_type;
+    s.ldy = w->rows;
+    if (stream_int_serves(s) && digit_bytes + 256 <= kStreamScratchBytes) {
+      QX_TRY(workspace->reserve(kWorkspaceCounterBytes + digit_bytes + 256));
+      uint8_t* scratch = static_cast<uint8_t*>(workspace->base) + kWorkspaceCounterBytes;
+      s.x = reinterpret_cast<const int8_t*>(scratch);
+      s.as = reinterpret_cast<const float*>(scratch + digit_bytes);
+      QX_TRY(launch_stream_digits(x, x_type, reinterpret_cast<int8_t*>(scratch),
+                                  reinterpret_cast<float*>(scratch + digit_bytes), m, w->columns, stream));
+      return launch_stream_int(s, stream);
+    }
+  }
+  if (stream_scaled_route(w, x_type, m)) {
+    StreamScaledArgs s{};
+    s.source = int8 ? kStreamBytes : kStreamNibbles;
+    s.codes = w->data;
+    s.scales = w->scales;
+    s.zeros = w->zeros;
+    s.nibble_xor = scaled.nibble_xor;
+    s.rows = w->rows;
+    s.columns = w->columns;
+    s.group = scaled.group;
+    s.x = x;
+    s.x_type = x_type;
+    s.order = w->act_order;
+    s.m = m;
+    s.bias = bias;
+    s.activation = activation;
+    s.y = y;
+    s.y_type = y_type;
+    s.ldy = w->rows;
+    const size_t stream_bytes = stream_scaled_scratch_bytes(s);
+    if (stream_scaled_serves(s) && stream_bytes <= kStreamScratchBytes) {
+      if (stream_bytes != 0) QX_TRY(workspace->reserve(kWorkspaceCounterBytes + stream_bytes));
+      return launch_stream_scaled(s, stream_bytes != 0 ? static_cast<uint8_t*>(workspace->base) + kWorkspaceCounterBytes : nullptr,
+                                  stream);
+    }
+  }
   if (scaled_route(w, x_type, m) && scaled_gemm_serves(scaled)) {
     const int sm_count = ctx->prop.multiProcessorCount;
     // (and what the digit kernels of smaller batches use)

@@ -25,6 +25,7 @@
 #include "qx_common.cuh"
 #include "qx_int8_gemm.cuh"
 #include "qx_scaled_gemm.cuh"
+#include "qx_stream_mma.cuh"
 
 namespace qx {
 namespace {
@@ -558,6 +559,40 @@ qx_status launch_w4a8_tensor(const uint8_t* packed, const float* weight_scales, 
   return launch_scaled_gemm(a, scratch, counters, kTensorCounterBytes, ctas, ctx->error_dev, stream);
 }
 
+// Where the codes are streamed past up to 64 rows (qx_stream_mma.cu; us, there | dp4a kernel, then | tensor_route):
+// rows on whole vectors: 4096 x 4096: 1 row 7.3 | 5.3, 2: 7.3 | 6.8, 16: 8.3 | 22.6, 14336 x 4096: 4: 14.2 | 24.9,
+// 16: 16.9 | 34.5, 64: 36.9 | 41.9, 2048 x 2048: 2: 5.1 | 4.3, 64: 9.7 | 24.7;
+// rows that start anywhere: 1024 x 1030: 1: 4.9 | 5.6, 5: 5.0 | 13.6;  4096 x 4094: 1: 9.2 | 21.3;  4096 x 4098:
+// 32: 12.6 | 25.7;  14336 x 8190: 8: 37.6 | 72.9, 40: 67.5 | 76.7;  4096 x 8190: 64: 29 | 42.6.
+bool stream_route(long long m, long long k) { return m <= kStreamColumns && (m > 2 || k % 32 != 0); }
+// Small batches: codes streamed past the activations (qx_stream_mma.cu). Scratch: [codes][scales][sums].
+qx_status launch_w4a8_stream(const uint8_t* packed, const float* weight_scales, const float* x, float* y,
+                             uint8_t* scratch, long long m, long long n, long long k, bool* served,
+                             cudaStream_t stream) {
+  int8_t* codes = reinterpret_cast<int8_t*>(scratch);
+  scratch += align_up(stream_code_bytes(m, k), 256);
+  float* scales = reinterpret_cast<float*>(scratch);
+  int* sums = reinterpret_cast<int*>(scratch + align_up(static_cast<size_t>(m) * 4, 256));
+  StreamIntArgs s{};
+  s.source = k % 16 == 0 && reinterpret_cast<uintptr_t>(packed) % 8 == 0 ? kStreamNibbles : kStreamNibblesLoose;
+  s.result = kStreamW4A8;
+  s.codes = packed;
+  s.x = codes;
+  s.x_rows = static_cast<int>(m);
+  s.rows = n;
+  s.columns = k;
+  s.ws = weight_scales;
+  s.as = scales;
+  s.zp = sums;
+  s.y = y;
+  s.y_type = QX_STORAGE_F32;
+  s.ldy = n;
+  *served = stream_int_serves(s);
+  if (!*served) return QX_STATUS_OK;
+  QX_TRY(launch_stream_codes(x, codes, scales, sums, m, k, stream));
+  return launch_stream_int(s, stream);
+}
+
 }  // namespace
 
 // y[m][n] from W4A8 operands already on the device (codes, scales, code sums of x).
@@ -687,6 +722,12 @@ qx_status qx_lowbit_gemm_w8a8_dev(const uint8_t* packed_dev, const float* weight
     return QX_STATUS_INVALID_SHAPE;
   }
   uint8_t* base = static_cast<uint8_t*>(scratch_dev);
+  if (stream_route(m, k) && reinterpret_cast<uintptr_t>(base) % 16 == 0) {
+    bool served = false;
+    QX_TRY(launch_w4a8_stream(packed_dev, weight_scales_dev, x_dev, y_dev, base, m, n, k, &served,
+                              static_cast<cudaStream_t>(stream)));
+    if (served) return QX_STATUS_OK;
+  }
   if (tensor_route(m, n, k) && reinterpret_cast<uintptr_t>(base) % 16 == 0) {
     bool served = false;
     QX_TRY(launch_w4a8_tensor(packed_dev, weight_scales_dev, x_dev, y_dev, base, m, n, k, &served,

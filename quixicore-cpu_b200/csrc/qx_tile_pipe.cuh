@@ -94,5 +94,32 @@ __device__ __forceinline__ uint32_t convert_bytes2(uint32_t w, uint32_t selector
   return sub2<false>(p, 0x64806480u);
 }
 
+// Eight nibbles -> eight 16-bit whole numbers nibble - z in column order. A nibble under the
+// exponent bits of `magic` (f16 1024 = 0x6400, bf16 128 times 2^-16: steps of one) is base + nibble;
+// `base_z` holds base + z twice.
+template <bool BF16>
+__device__ __forceinline__ uint4 convert_nibbles(uint32_t w, uint32_t base_z) {
+  const uint32_t magic = BF16 ? kBf16Base * 0x10001u : 0x64006400u;
+  const uint32_t high = w >> 4;
+  uint32_t out[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t pair = __byte_perm(w, high, i | (i << 4) | ((4 + i) << 8) | ((4 + i) << 12));
+    out[i] = sub2<BF16>((pair & 0x000F000Fu) | magic, base_z);
+  }
+  return make_uint4(out[0], out[1], out[2], out[3]);
+}
+// z as it is subtracted: (base + z) twice
+template <bool BF16>
+__device__ __forceinline__ uint32_t zero_word(float z) {
+  uint32_t bits;
+  if (BF16) {
+    bits = __float_as_uint((128.0f + z) / kBf16Unscale) >> 16;  // exact: 128 .. 143
+  } else {
+    bits = __half_as_ushort(__float2half_rn(1024.0f + z));
+  }
+  return bits | (bits << 16);
+}
+
 }  // namespace tile
 }  // namespace qx
