@@ -194,19 +194,31 @@ def _np(a):
     if a is None:
         return None
     assert isinstance(a, np.ndarray) and a.flags["C_CONTIGUOUS"], "need a contiguous numpy array"
-    return a.ctypes.data_as(_vp)
+    return a.ctypes.data  # (the argument's declared type makes a pointer of it)
 
 
 def _dev(t):
     if t is None:
         return None
     assert t.is_cuda and t.is_contiguous(), "need a contiguous CUDA tensor"
-    return _vp(t.data_ptr())
+    return t.data_ptr()
 
 
 def _stream():
-    import torch
-    return _vp(torch.cuda.current_stream().cuda_stream)
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+        # the handle itself: a Stream object per call is a microsecond of a call's ten
+        stream, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+        torch.cuda.current_stream()  # (initialises CUDA)
+        if stream is not None and device is not None:
+            _raw_stream = lambda: stream(device())
+        else:
+            _raw_stream = lambda: torch.cuda.current_stream().cuda_stream
+    return _raw_stream()
+
+
+_raw_stream = None
 
 
 def last_error() -> str:
@@ -387,19 +399,19 @@ class PackedWeights:
 
     # host buffers (numpy): the reference-facing call
     def qgemm_prepacked(self, x, m, y=None):
-        rows = self.info()["rows"] if self.handle else 0
         if y is None:
+            rows = self.info()["rows"] if self.handle else 0
             y = np.zeros((m, max(rows, 1)), np.float32)
         return lib.qx_qgemm_prepacked(self.handle, _np(x), _np(y), m, None), y
 
     # raw host pointers (e.g. pinned torch tensors): the end-to-end timed call
     def qgemm_prepacked_ptr(self, x_ptr, y_ptr, m) -> int:
-        return lib.qx_qgemm_prepacked(self.handle, _vp(x_ptr), _vp(y_ptr), m, None)
+        return lib.qx_qgemm_prepacked(self.handle, x_ptr, y_ptr, m, None)
 
     # device tensors, torch's current stream
     def qgemm_dev(self, x, y, m, ldy=None) -> int:
         ldy = y.shape[-1] if ldy is None else ldy
-        return lib.qx_qgemm_prepacked_dev(self.handle, _dev(x), _vp(y.data_ptr()), m, ldy, None,
+        return lib.qx_qgemm_prepacked_dev(self.handle, _dev(x), y.data_ptr(), m, ldy, None,
                                           _stream())
 
     def prepare_fused(self, fmt, parts, rows, columns) -> int:
@@ -416,21 +428,21 @@ class PackedWeights:
         return lib.qx_qgemm_fused_dev(self.handle, _dev(x), pointers, m, None, _stream())
 
     def up_gate_activation_dev(self, x, out, scratch, gelu_tanh=True) -> int:
-        return lib.qx_qgemv_up_gate_activation_dev(self.handle, _dev(x), _vp(out.data_ptr()),
-                                                   _vp(scratch.data_ptr()), 1 if gelu_tanh else 0,
+        return lib.qx_qgemv_up_gate_activation_dev(self.handle, _dev(x), out.data_ptr(),
+                                                   scratch.data_ptr(), 1 if gelu_tanh else 0,
                                                    None, _stream())
 
     def qgemv_w8a8_dev(self, x, y) -> int:
-        return lib.qx_qgemv_w8a8_prepacked_dev(self.handle, _dev(x), _vp(y.data_ptr()), None, _stream())
+        return lib.qx_qgemv_w8a8_prepacked_dev(self.handle, _dev(x), y.data_ptr(), None, _stream())
 
     def qgemv_noalloc_dev(self, x, y) -> int:
         """Decode GEMV through the entry point that never allocates device memory."""
-        return lib.qx_qgemv_prepacked_noalloc_dev(self.handle, _dev(x), _vp(y.data_ptr()),
+        return lib.qx_qgemv_prepacked_noalloc_dev(self.handle, _dev(x), y.data_ptr(),
                                                   _stream())
 
     def qgemm_bf16_dev(self, x_bf16, y, m, ldy=None) -> int:
         ldy = y.shape[-1] if ldy is None else ldy
-        return lib.qx_qgemm_prepacked_bf16_dev(self.handle, _dev(x_bf16), _vp(y.data_ptr()), m,
+        return lib.qx_qgemm_prepacked_bf16_dev(self.handle, _dev(x_bf16), y.data_ptr(), m,
                                                ldy, None, _stream())
 
 
@@ -500,7 +512,7 @@ class CanonicalWeights:
 
     def qgemm_storage_dev(self, x, x_type, y, y_type, m, bias=None, activation=ACT_NONE) -> int:
         return lib.qx_qgemm_prepacked_epilogue_storage_dev(
-            self.handle, _vp(x.data_ptr()), x_type, _dev(bias), _vp(y.data_ptr()), y_type, m,
+            self.handle, x.data_ptr(), x_type, _dev(bias), y.data_ptr(), y_type, m,
             activation, None, _stream())
 
 
@@ -585,12 +597,12 @@ def int8_gemm_dev(w, x, ws, xs, y, m, n, k, row_sum=None, zp=None, acc=None, ldy
                   check_scales=False) -> int:
     ldy = n if ldy is None else ldy
     return lib.qx_int8_gemm_dev(_dev(w), _dev(x), _dev(ws), _dev(xs), _dev(row_sum), _dev(zp),
-                                _vp(y.data_ptr()), _dev(acc), m, n, k, ldy,
+                                y.data_ptr(), _dev(acc), m, n, k, ldy,
                                 1 if row_sum is not None else 0, 1 if check_scales else 0,
                                 _stream())
 
 
 def qgemm_w8a32_dev(w, ws, x, y, m, n, k, ldy=None, check_scales=False) -> int:
     ldy = n if ldy is None else ldy
-    return lib.qx_qgemm_w8a32_dev(_dev(w), _dev(ws), _dev(x), _vp(y.data_ptr()), m, n, k, ldy,
+    return lib.qx_qgemm_w8a32_dev(_dev(w), _dev(ws), _dev(x), y.data_ptr(), m, n, k, ldy,
                                   1 if check_scales else 0, None, _stream())

@@ -54,21 +54,32 @@ __global__ void __launch_bounds__(256) stage_in_kernel(const uint4* __restrict__
   const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < n16) dst[i] = src[i];
 }
-qx_status stage_in(void* dst, const void* src, size_t bytes, cudaStream_t s) {
-  constexpr size_t kLimit = 256 * 1024;
-  if (bytes > 0 && bytes <= kLimit && bytes % 16 == 0 &&
-      reinterpret_cast<uintptr_t>(src) % 16 == 0 && reinterpret_cast<uintptr_t>(dst) % 16 == 0) {
-    cudaPointerAttributes attributes{};
-    if (cudaPointerGetAttributes(&attributes, src) == cudaSuccess &&
-        attributes.type == cudaMemoryTypeHost && attributes.devicePointer != nullptr) {
-      const size_t n16 = bytes / 16;
-      stage_in_kernel<<<static_cast<unsigned>((n16 + 255) / 256), 256, 0, s>>>(
-          static_cast<const uint4*>(attributes.devicePointer), static_cast<uint4*>(dst), n16);
-      count_launch();
-      QX_CUDA_TRY(cudaGetLastError());
-      return QX_STATUS_OK;
+// The address at which the GPU reaches host memory that is pinned or registered, else null.
+void* device_address(const void* host) {
+  cudaPointerAttributes attributes{};
+  if (cudaPointerGetAttributes(&attributes, host) == cudaSuccess && attributes.type == cudaMemoryTypeHost) {
+    return attributes.devicePointer;
+  }
+  (void)cudaGetLastError();  // unregistered host memory is not an error here
+  return nullptr;
+}
+// Small inputs in pageable memory take the same way through the context's pinned memory (its mutex is
+// held, and the call before has waited for its kernels).
+qx_status stage_in(DeviceContext* ctx, void* dst, const void* src, size_t bytes) {
+  const cudaStream_t s = ctx->stream;
+  if (bytes > 0 && bytes <= kBounceBytes && bytes % 16 == 0 && reinterpret_cast<uintptr_t>(dst) % 16 == 0) {
+    const void* from = reinterpret_cast<uintptr_t>(src) % 16 == 0 ? device_address(src) : nullptr;
+    if (from == nullptr) {
+      QX_TRY(ctx->ensure_bounce());
+      std::memcpy(ctx->bounce_host, src, bytes);
+      from = ctx->bounce_dev;
     }
-    (void)cudaGetLastError();  // unregistered host memory is not an error here
+    const size_t n16 = bytes / 16;
+    stage_in_kernel<<<static_cast<unsigned>((n16 + 255) / 256), 256, 0, s>>>(static_cast<const uint4*>(from),
+                                                                              static_cast<uint4*>(dst), n16);
+    count_launch();
+    QX_CUDA_TRY(cudaGetLastError());
+    return QX_STATUS_OK;
   }
   return h2d(dst, src, bytes, s);
 }
@@ -439,25 +450,30 @@ qx_status qx_qgemm_prepacked(const qx_weights* weights, const float* x, float* y
   const size_t y_bytes = static_cast<size_t>(m) * weights->rows * sizeof(float);
   const size_t off_x = st.add(x_bytes), off_y = st.add(y_bytes);
   QX_TRY(ctx->ensure_staging(st.offset));
-  QX_TRY(stage_in(st.at(off_x), x, x_bytes, ctx->stream));
+  QX_TRY(stage_in(ctx, st.at(off_x), x, x_bytes));
   // Results go straight to the caller's buffer when the GPU can address it (pinned or
   // registered host memory): the kernel's row finishers write it over PCIe and the copy
-  // back is saved. Pageable memory takes the staged copy.
-  float* y_target = reinterpret_cast<float*>(st.at(off_y));
-  bool direct = false;
-  cudaPointerAttributes attributes{};
-  if (cudaPointerGetAttributes(&attributes, y) == cudaSuccess &&
-      attributes.type == cudaMemoryTypeHost && attributes.devicePointer != nullptr) {
-    y_target = static_cast<float*>(attributes.devicePointer);
-    direct = true;
-  } else {
-    (void)cudaGetLastError();  // unregistered host memory is not an error here
+  // back is saved. Small ones in pageable memory go to the context's pinned memory that way and
+  // from there by the CPU; larger ones take the staged copy.
+  float* y_target = static_cast<float*>(device_address(y));
+  const bool direct = y_target != nullptr, bounced = !direct && y_bytes <= kBounceBytes;
+  if (bounced) {
+    QX_TRY(ctx->ensure_bounce());
+    y_target = reinterpret_cast<float*>(ctx->bounce_dev + kBounceBytes);
+  } else if (!direct) {
+    y_target = reinterpret_cast<float*>(st.at(off_y));
   }
-  QX_TRY(launch_qgemm_f32(weights, reinterpret_cast<const float*>(st.at(off_x)), y_target, m,
-                          weights->rows, workspace != nullptr ? workspace : &ctx->workspace,
-                          ctx->stream));
-  if (!direct) QX_TRY(d2h(y, st.at(off_y), y_bytes, ctx->stream));
-  return sync_and_check(ctx, ctx->stream);
+  const qx_status launched = launch_qgemm_f32(weights, reinterpret_cast<const float*>(st.at(off_x)), y_target, m,
+                                              weights->rows, workspace != nullptr ? workspace : &ctx->workspace,
+                                              ctx->stream);
+  if (launched != QX_STATUS_OK) {
+    (void)cudaStreamSynchronize(ctx->stream);  // (the pinned memory may still be read)
+    return launched;
+  }
+  if (!direct && !bounced) QX_TRY(d2h(y, st.at(off_y), y_bytes, ctx->stream));
+  QX_TRY(sync_and_check(ctx, ctx->stream));
+  if (bounced) std::memcpy(y, ctx->bounce_host + kBounceBytes, y_bytes);
+  return QX_STATUS_OK;
 }
 
 qx_status qx_qgemm_prepacked_dev(const qx_weights* weights, const float* x_dev, float* y_dev,

@@ -60,6 +60,8 @@ struct qx_workspace {
 
 namespace qx {
 
+constexpr size_t kBounceBytes = 256 * 1024;  // one way
+
 struct DeviceContext {
   int device = -1;
   cudaDeviceProp prop{};
@@ -69,6 +71,12 @@ struct DeviceContext {
   // staging buffers for host-pointer calls (grow-only)
   void* staging = nullptr;
   size_t staging_bytes = 0;
+  // Pinned memory that small operands in pageable host memory pass through (kBounceBytes each way,
+  // allocated with the first such call): a copy by the CPU and a kernel's read or write of it take a
+  // third of the time of the runtime's own pageable copies.
+  uint8_t* bounce_host = nullptr;
+  uint8_t* bounce_dev = nullptr;  // the same as the GPU addresses it
+  qx_status ensure_bounce();
   int* flag = nullptr;            // device word for scale / finiteness checks
   // Error word of the tensor-core kernels (a bounded wait that gave up leaves its role code
   // there): pinned host memory the GPU can address, written only on that path, so the host

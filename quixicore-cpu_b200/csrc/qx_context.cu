@@ -42,6 +42,21 @@ qx_status DeviceContext::ensure_staging(size_t bytes) {
   return QX_STATUS_OK;
 }
 
+qx_status DeviceContext::ensure_bounce() {
+  if (bounce_host != nullptr) return QX_STATUS_OK;
+  void* host = nullptr;
+  void* dev = nullptr;
+  QX_CUDA_TRY(cudaHostAlloc(&host, 2 * kBounceBytes, cudaHostAllocMapped));
+  const cudaError_t mapped = cudaHostGetDevicePointer(&dev, host, 0);
+  if (mapped != cudaSuccess) {
+    (void)cudaFreeHost(host);
+    QX_CUDA_TRY(mapped);
+  }
+  bounce_host = static_cast<uint8_t*>(host);
+  bounce_dev = static_cast<uint8_t*>(dev);
+  return QX_STATUS_OK;
+}
+
 qx_status current_context(DeviceContext** out) {
   int device = -1;
   int count = 0;
