@@ -82,8 +82,7 @@ namespace {
 
 constexpr int kBM = 128;        // output channels per tile (MMA M, TMEM lanes)
 constexpr int kBK = 128;        // bytes of K per pipeline stage (one swizzle atom)
-constexpr int kMaxStages = 4;
-__host__ __device__ constexpr int stages_for(int na) { return na == 1 ? 4 : 3; }
+constexpr int kMaxStages = 8;
 constexpr int kEpiWarps = 8;  // two per TMEM lane quarter, splitting the token columns
 constexpr int kThreads = 64 + 32 * kEpiWarps;
 constexpr int kTmemCols = 512;  // two accumulators of up to 256 columns
@@ -98,6 +97,7 @@ struct TcParams {
   long long m, n, ldy;
   int k_slabs;   // ceil(k / 128)
   int bn;        // tokens per tile: multiple of 32, <= 256
+  int stages;    // K-slabs in flight
   int o_tiles, r_tiles;
   int asymmetric;
   int stream_k;        // 1: contiguous (tile, K-slab) ranges per CTA; 0: whole tiles round robin
@@ -164,7 +164,6 @@ __global__ void __launch_bounds__(kThreads, 1) int8_gemm_tc_kernel(
     const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
     const TcParams p) {
   constexpr uint32_t kAccBuffers = NA == 1 ? 2 : 1;
-  constexpr int kStages = stages_for(NA);
   using namespace sm100;
   extern __shared__ uint8_t smem_raw[];
   // stage ring, 1024-byte aligned for the 128-byte swizzle
@@ -173,7 +172,8 @@ __global__ void __launch_bounds__(kThreads, 1) int8_gemm_tc_kernel(
   const uint32_t a_bytes = NA * kBM * kBK;
   const uint32_t b_bytes = static_cast<uint32_t>(p.bn) * kBK;
   const uint32_t stage_bytes = a_bytes + b_bytes;
-  TcBarriers* bars = reinterpret_cast<TcBarriers*>(smem + kStages * stage_bytes);
+  const uint32_t stages = static_cast<uint32_t>(p.stages);
+  TcBarriers* bars = reinterpret_cast<TcBarriers*>(smem + stages * stage_bytes);
   float* as_tile = reinterpret_cast<float*>(bars + 1);  // [2][256] activation scales
   int* zp_tile = reinterpret_cast<int*>(as_tile + 2 * 256);
 
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kThreads, 1) int8_gemm_tc_kernel(
   volatile int* abort_flag = &bars->abort_flag;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < kMaxStages; ++s) {
       mbar_init(&bars->full[s], 1);
       mbar_init(&bars->empty[s], 1);
     }
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(kThreads, 1) int8_gemm_tc_kernel(
           mbar_arrive_expect_tx(&bars->full[stage], stage_bytes);
           tma_load_2d(sa, &map_w, &bars->full[stage], ks * kBK, o0);
           tma_load_2d(sa + a_bytes, &map_x, &bars->full[stage], ks * kBK, r0);
-          if (++stage == kStages) {
+          if (++stage == stages) {
             stage = 0;
             phase ^= 1u;
           }
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(kThreads, 1) int8_gemm_tc_kernel(
             }
           }
           tc_commit(&bars->empty[stage]);  // frees the slab once the MMAs have read it
-          if (++stage == kStages) {
+          if (++stage == stages) {
             stage = 0;
             phase ^= 1u;
           }
@@ -475,9 +475,13 @@ __global__ void __launch_bounds__(kThreads, 1) int8_gemm_tc_kernel(
   }
 }
 
-size_t tc_smem_bytes(int na, int bn) {
-  return 1024 + static_cast<size_t>(stages_for(na)) * (na * kBM * kBK + bn * kBK) + sizeof(TcBarriers) +
-         2 * 256 * sizeof(float) + 2 * 256 * sizeof(int) + 16 + 64;
+constexpr size_t kSmemMax = 227 * 1024;
+constexpr size_t kTablesBytes = 1024 + sizeof(TcBarriers) + 2 * 256 * sizeof(float) + 2 * 256 * sizeof(int) + 16 + 64;
+constexpr size_t tc_stage_bytes(int na, int bn) { return static_cast<size_t>(na * kBM + bn) * kBK; }
+// as many K-slabs in flight as fit: 3 of the largest tile, 8 of small ones, whose slabs are quickly used up
+int tc_stages(int na, int bn) {
+  const size_t fit = (kSmemMax - kTablesBytes) / tc_stage_bytes(na, bn);
+  return fit > kMaxStages ? kMaxStages : static_cast<int>(fit);
 }
 
 }  // namespace
@@ -494,14 +498,14 @@ template <int NA>
 qx_status launch_tc_na(const CUtensorMap& map_w, const CUtensorMap& map_x, const TcParams& p,
                        int grid, cudaStream_t stream) {
   static SmemOptIn opt_in;
-  QX_TRY(opt_in.ensure(int8_gemm_tc_kernel<NA>, tc_smem_bytes(NA, 256)));
+  QX_TRY(opt_in.ensure(int8_gemm_tc_kernel<NA>, kSmemMax));
   cudaLaunchAttribute attribute{};
   attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t config{};
   config.gridDim = dim3(static_cast<unsigned>(grid));
   config.blockDim = dim3(kThreads);
-  config.dynamicSmemBytes = tc_smem_bytes(NA, p.bn);
+  config.dynamicSmemBytes = kTablesBytes + p.stages * tc_stage_bytes(NA, p.bn);
   config.stream = stream;
   config.attrs = &attribute;
   config.numAttrs = 1;
@@ -557,28 +561,59 @@ bool choose_stream_k(long long tiles128, int k_slabs, int sm_count) {
   return tiles128 * k_slabs >= sm_count && tiles128 <= kStreamKMaxTiles;
 }
 
-// weight tiles per CTA tile: 2 (256 channels) when that still gives most SMs a tile
-int choose_weight_tiles(long long n, long long r_tiles, int sm_count) {
+// A tile's channels (na tiles of 128) and tokens: the pair for which the slowest SM is done first. Cycles of a
+// 32-byte step of K: what shared memory has to take in and give out at 128 bytes a cycle, (na * 128 + bn) rows
+// fetched and na * (128 + bn) read, above the tensor pipe's na * bn / 2 for every tile; and no less than the 100 at which a
+// ring of small slabs still hides the fetches. The results of an SM's last tile are stored with nothing beside them.
+// Measured (us, chosen here | 256 tokens and 256 channels wherever they gave six of ten SMs a tile): 200 rows 2048 x 8192
+// 15.2 | 30.9, 512 rows 1024 x 4096 7.0 | 13.7, 128 rows 4096 x 4096 7.7 | 11.6, 300 rows 14336 x 4096 26.4 | 37.4, 1300 rows
+// 9000 x 2048 29.2 | 41.3, 2048 rows 1024 x 1024 5.1 | 7.2; 512 rows 14336 x 4096 30.0 either way.
+struct TileChoice {
+  int na, bn;
+};
+TileChoice choose_tile(long long m, long long n, long long k, int sm_count) {
+  int forced_na = 0;
   if (const char* forced = std::getenv("QX_B200_INT8_WEIGHT_TILES")) {
-    if (forced[0] == '1') return 1;
-    if (forced[0] == '2') return 2;
+    if (forced[0] == '1' || forced[0] == '2') forced_na = forced[0] - '0';
   }
-  const long long tiles2 = (n + 2 * kBM - 1) / (2 * kBM) * r_tiles;
-  return tiles2 * 10 >= static_cast<long long>(sm_count) * 6 ? 2 : 1;
+  const long long steps = (k + 31) / 32;
+  TileChoice best{1, 32};
+  long long best_cycles = -1;
+  for (int na = 1; na <= 2; ++na) {
+    if (forced_na != 0 && na != forced_na) continue;
+    for (int bn = 256; bn >= 32; bn -= 32) {
+      if (bn > 32 && bn - 32 >= m) continue;  // (nothing but padding in the last 32)
+      const long long tiles = (n + na * kBM - 1) / (na * kBM) * ((m + bn - 1) / bn);
+      const long long rounds = (tiles + sm_count - 1) / sm_count;
+      const long long moved = (na * 128 + bn + na * (128 + bn)) / 4;
+      const long long cycles = rounds * steps * (moved > 100 ? moved : 100) + 6LL * na * bn;
+      if (best_cycles < 0 || cycles < best_cycles) {
+        best_cycles = cycles;
+        best = TileChoice{na, bn};
+      }
+    }
+  }
+  return best;
 }
 }  // namespace
 
 qx_status launch_int8_gemm_tc(const Int8GemmArgs& a, cudaStream_t stream) {
   DeviceContext* ctx = nullptr;
   QX_TRY(current_context(&ctx));
-  int bn = 256;
-  if (a.m < 256) bn = static_cast<int>((a.m + 31) / 32 * 32);
-  const long long r_tiles = (a.m + bn - 1) / bn;
   const int k_slabs = static_cast<int>((a.k + kBK - 1) / kBK);
   const int sm_count = ctx->prop.multiProcessorCount;
+  int bn = 256;
+  if (a.m < 256) bn = static_cast<int>((a.m + 31) / 32 * 32);
+  long long r_tiles = (a.m + bn - 1) / bn;
   const bool stream_k = sm_count <= kStreamKMaxCtas &&
                         choose_stream_k((a.n + kBM - 1) / kBM * r_tiles, k_slabs, sm_count);
-  const int na = stream_k ? 1 : choose_weight_tiles(a.n, r_tiles, sm_count);
+  int na = 1;
+  if (!stream_k) {
+    const TileChoice tile = choose_tile(a.m, a.n, a.k, sm_count);
+    na = tile.na;
+    bn = tile.bn;
+    r_tiles = (a.m + bn - 1) / bn;
+  }
   CUtensorMap map_w, map_x;
   if (!encode_tma_2d(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.w, static_cast<uint64_t>(a.k),
                      static_cast<uint64_t>(a.n), static_cast<uint64_t>(a.k), kBK,
@@ -601,6 +636,7 @@ qx_status launch_int8_gemm_tc(const Int8GemmArgs& a, cudaStream_t stream) {
   p.ldy = a.ldy;
   p.k_slabs = static_cast<int>((a.k + kBK - 1) / kBK);
   p.bn = bn;
+  p.stages = tc_stages(na, bn);
   p.o_tiles = static_cast<int>((a.n + na * kBM - 1) / (na * kBM));
   p.r_tiles = static_cast<int>(r_tiles);
   p.asymmetric = a.asymmetric ? 1 : 0;
