@@ -862,6 +862,9 @@ constexpr int kPlanes = 4;
 __global__ void __launch_bounds__(256) canonical_row_digits_kernel(
     const void* __restrict__ x, int x_type, long long columns, long long chunk_tokens,
     int8_t* __restrict__ planes, float* __restrict__ plane_scale) {
+  // (behind the kernel in front: the activations may be its output, and the product in front reads the planes)
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   __shared__ float warp_max[8];
   const long long token = blockIdx.x;
   const long long base = token * columns;
@@ -917,6 +920,8 @@ __global__ void __launch_bounds__(256) canonical_row_digits_kernel(
 __global__ void __launch_bounds__(256) canonical_combine_kernel(
     const float* __restrict__ partial, long long chunk_tokens, long long tokens, long long rows,
     long long ldy, const float* __restrict__ bias, int activation, void* __restrict__ y, int y_type) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const long long total = tokens * rows;
   const long long plane = chunk_tokens * rows;
   for (long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x; i < total;
@@ -938,6 +943,23 @@ size_t prefill_scratch_bytes(long long m, long long rows, long long columns) {
          static_cast<size_t>(kPlanes * chunk * rows) * sizeof(float);
 }
 
+// Launch of 256 threads per CTA that may begin while the kernel in front still runs; the kernel waits for it itself.
+template <class... Params, class... Args>
+qx_status launch_programmatic(void (*kernel)(Params...), dim3 grid, cudaStream_t stream, Args... args) {
+  cudaLaunchAttribute attribute{};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = grid;
+  config.blockDim = dim3(256);
+  config.stream = stream;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  QX_CUDA_TRY(cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...));
+  count_launch();
+  return QX_STATUS_OK;
+}
+
 qx_status launch_prefill_int8(const CanonicalParams& p, uint8_t* scratch, int sm_count,
                               cudaStream_t stream) {
   const long long chunk = p.m < kPrefillChunk ? p.m : kPrefillChunk;
@@ -952,46 +974,27 @@ qx_status launch_prefill_int8(const CanonicalParams& p, uint8_t* scratch, int sm
     const long long wanted = (2LL * sm_count + tokens - 1) / tokens;
     const long long most = (p.columns + 1023) / 1024;
     const unsigned splits = static_cast<unsigned>(wanted < 1 ? 1 : (wanted > most ? most : (wanted > 16 ? 16 : wanted)));
-    canonical_row_digits_kernel<<<dim3(static_cast<unsigned>(tokens), splits), 256, 0, stream>>>(
-        x, p.x_type, p.columns, chunk, planes, plane_scale);
-    count_launch();
-    QX_CUDA_TRY(cudaGetLastError());
-    if (tokens < chunk) {
-      // the planes of a short last chunk are not contiguous token rows: run them one by one
-      for (int d = 0; d < kPlanes; ++d) {
-        Int8GemmArgs a{};
-        a.w = reinterpret_cast<const int8_t*>(p.data);
-        a.x = planes + d * chunk * p.columns;
-        a.ws = p.scales;
-        a.as = plane_scale + d * chunk;
-        a.y = partial + d * chunk * p.rows;
-        a.m = tokens;
-        a.n = p.rows;
-        a.k = p.columns;
-        a.ldy = p.rows;
-        QX_TRY(launch_int8_gemm(a, stream));
-      }
-    } else {
-      Int8GemmArgs a{};
-      a.w = reinterpret_cast<const int8_t*>(p.data);
-      a.x = planes;
-      a.ws = p.scales;
-      a.as = plane_scale;
-      a.y = partial;
-      a.m = kPlanes * chunk;
-      a.n = p.rows;
-      a.k = p.columns;
-      a.ldy = p.rows;
-      QX_TRY(launch_int8_gemm(a, stream));
-    }
+    // (the planes of a chunk are its own tokens apart, so that those of a short last one are rows of one product
+    // as well: 300 tokens on 4096 x 4096 70 us with a product per plane)
+    QX_TRY(launch_programmatic(canonical_row_digits_kernel, dim3(static_cast<unsigned>(tokens), splits), stream, x, p.x_type,
+                               p.columns, tokens, planes, plane_scale));
+    Int8GemmArgs a{};
+    a.w = reinterpret_cast<const int8_t*>(p.data);
+    a.x = planes;
+    a.ws = p.scales;
+    a.as = plane_scale;
+    a.y = partial;
+    a.m = kPlanes * tokens;
+    a.n = p.rows;
+    a.k = p.columns;
+    a.ldy = p.rows;
+    QX_TRY(launch_int8_gemm(a, stream));
     uint8_t* y = static_cast<uint8_t*>(p.y) + static_cast<size_t>(t0 * p.ldy) * y_bytes;
     const long long total = tokens * p.rows;
     const long long blocks = (total + 255) / 256;
     const long long cap = 8LL * sm_count;
-    canonical_combine_kernel<<<static_cast<unsigned>(blocks < cap ? blocks : cap), 256, 0, stream>>>(
-        partial, chunk, tokens, p.rows, p.ldy, p.bias, p.activation, y, p.y_type);
-    count_launch();
-    QX_CUDA_TRY(cudaGetLastError());
+    QX_TRY(launch_programmatic(canonical_combine_kernel, dim3(static_cast<unsigned>(blocks < cap ? blocks : cap)), stream,
+                               partial, tokens, tokens, p.rows, p.ldy, p.bias, p.activation, y, p.y_type));
   }
   return QX_STATUS_OK;
 }
