@@ -447,6 +447,7 @@ __global__ void __launch_bounds__(kThreads, CTAS) stream_scaled_kernel(const Sca
       for (int c = 0; c < 4; ++c) part[i][n][c] = sum[i][n][c] = 0.0f;
     }
   }
+  const uint32_t base_x = (BF16 ? tile::kBf16Base * 0x10001u : 0x64006400u) ^ (p.nibble_xor & 0x000F000Fu);
   int until_flush = p.flush_steps - (s0 & (p.flush_steps - 1));
   // Two levels of sums: chains of four multiply-adds in registers, and the chains in the warp's own part of
   // `red`, so that a result is no further from float64 than those of the kernels for other batches
@@ -518,7 +519,8 @@ __global__ void __launch_bounds__(kThreads, CTAS) stream_scaled_kernel(const Sca
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
               if constexpr (kNibbles) {
-                const uint4 v = tile::convert_nibbles<BF16>(ring[d][i][h][q] ^ p.nibble_xor, base_z[i][h]);
+                const uint4 v = FRAGMENTS ? tile::convert_nibbles_apart<BF16>(ring[d][i][h][q], base_x, base_z[i][h])
+                                          : tile::convert_nibbles<BF16>(ring[d][i][h][q] ^ p.nibble_xor, base_z[i][h]);
                 a[i][h][0] = v.x;
                 a[i][h][1] = v.y;
                 a[i][h][2] = v.z;
@@ -658,12 +660,13 @@ __device__ __forceinline__ long long fragment_byte(long long c, long long column
 }
 
 // 16-bit activations in that order: [step][eight columns of a lane][plane][column tile][lane]; f32 ones as
-// three bf16 planes, each the truncated remainder of the ones before, so that their sum is the value.
+// three bf16 planes, each the truncated remainder of the ones before, so that their sum is the value. `apart`: the eight
+// columns as convert_nibbles_apart has them.
 template <int PLANES>
 __global__ void __launch_bounds__(256) stream_fragments_kernel(const void* __restrict__ x, int x_type,
                                                                const int* __restrict__ order, uint4* __restrict__ out,
                                                                int columns, int m, int lane_columns, int column_tiles,
-                                                               int total, int vector) {
+                                                               int total, int vector, int apart) {
   launch_dependents();  // (the projection's weights are prepared ones)
   wait_for_kernel_in_front();
   const int i = blockIdx.x * 256 + threadIdx.x;
@@ -677,7 +680,9 @@ __global__ void __launch_bounds__(256) stream_fragments_kernel(const void* __res
   uint32_t words[PLANES][4];
   if (PLANES == 1 && order == nullptr && vector != 0 && count >= 8) {
     const uint4 v = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(x) + base + column);
-    out[i] = v;
+    out[i] = apart != 0 ? make_uint4(__byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632),
+                                     __byte_perm(v.y, v.w, 0x5410), __byte_perm(v.y, v.w, 0x7632))
+                        : v;
     return;
   }
 #pragma unroll
@@ -686,7 +691,7 @@ __global__ void __launch_bounds__(256) stream_fragments_kernel(const void* __res
     for (int plane = 0; plane < PLANES; ++plane) words[plane][j] = 0u;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int k = 2 * j + h;
+      const int k = apart != 0 ? j + 4 * h : 2 * j + h;
       if (k < count) {
         const long long from = base + (order != nullptr ? order[column + k] : column + k);
         if (PLANES == 3) {
@@ -973,7 +978,7 @@ qx_status launch_stream_scaled(const StreamScaledArgs& a, void* scratch, cudaStr
     const int vector = a.columns % 8 == 0 && reinterpret_cast<uintptr_t>(a.x) % 16 == 0 ? 1 : 0;
     QX_TRY(launch(planes == 3 ? stream_fragments_kernel<3> : stream_fragments_kernel<1>, (total + 255) / 256, 256, stream,
                   a.x, a.x_type, a.order, static_cast<uint4*>(scratch), static_cast<int>(a.columns),
-                  static_cast<int>(a.m), step / 4, tiles, total, vector));
+                  static_cast<int>(a.m), step / 4, tiles, total, vector, a.source == kStreamNibbles ? 1 : 0));
   }
   p.codes = a.codes;
   p.scales = a.scales;

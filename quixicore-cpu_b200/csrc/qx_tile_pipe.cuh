@@ -109,6 +109,14 @@ __device__ __forceinline__ uint4 convert_nibbles(uint32_t w, uint32_t base_z) {
   }
   return make_uint4(out[0], out[1], out[2], out[3]);
 }
+// The same in the order (0, 4), (1, 5), (2, 6), (3, 7), which needs no byte permutes (those run at half rate);
+// `base_x` is the base's bits with the nibbles' exclusive-or in them, twice.
+template <bool BF16>
+__device__ __forceinline__ uint4 convert_nibbles_apart(uint32_t w, uint32_t base_x, uint32_t base_z) {
+  return make_uint4(sub2<BF16>((w & 0x000F000Fu) ^ base_x, base_z), sub2<BF16>(((w >> 4) & 0x000F000Fu) ^ base_x, base_z),
+                    sub2<BF16>(((w >> 8) & 0x000F000Fu) ^ base_x, base_z),
+                    sub2<BF16>(((w >> 12) & 0x000F000Fu) ^ base_x, base_z));
+}
 // z as it is subtracted: (base + z) twice
 template <bool BF16>
 __device__ __forceinline__ uint32_t zero_word(float z) {
