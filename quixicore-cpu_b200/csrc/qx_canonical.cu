@@ -25,6 +25,8 @@
 //           multiply-adds on exactly converted codes, every weight decoded on its own as in
 //           the reference (scale * code, or scale * (nibble - zero)).
 // With an act-order map the activations are first gathered into packed column order.
+//   streamed small batches (qx_stream_mma.cu, chosen by stream_digits_route and stream_scaled_route below): up to 16 tokens of
+//           int8 tensors with one scale per row, five to 32 of the others;
 //   tensor cores (int8 with one scale per row, five tokens or more): four digit planes under a
 //           per-token envelope through the W8A8 GEMM; see "long prefills" below.
 //   tensor cores with scales applied per group (batches of the 4-bit and group-scaled tensors):
@@ -40,11 +42,9 @@
 // bytes. The digit images of a call's activations (1792 bytes per token and 512 columns)
 // live in the device's default workspace.
 //
-// Kernels. CUDA cores for decode-sized batches, the tcgen05 W8A8 GEMM for int8 prefills.
-// Measured on 14336 x 4096 int8 with one bf16 token: 17 us per call for both launches (the
-// digit kernel and the projection behind it), 3.4 TB/s of the weights' bytes, about half of
-// the measured copy bandwidth; the float path ran the same shape in 24 us at 10 instructions
-// per weight, bound by instruction issue.
+// Kernels. CUDA cores and warp-level MMAs for decode-sized batches, the tcgen05 W8A8 GEMM for int8 prefills.
+// Measured on 14336 x 4096 int8 with one bf16 token: 15.6 us per call for both launches (digits and the projection behind
+// them), 17.2 on the dp4a digit kernels, 24 on the float path.
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -1045,7 +1045,7 @@ bool scaled_route(const qx_canonical_weights* w, int x_type, long long m) {
 //   int8, one scale per row (four digit rows per token, exact sums): 14336 x 4096: 1 token 15.6 | 17.2, 4: 17.2 | 34.2,
 //     8: 20.6 | 20.7 (and one launch less);  4096 x 4096: 1: 6.0 | 6.8, 8: 8.2 | 12.6, 12: 9.9 | 15.2;  8192 x 4096:
 //     8: 10.9 | 17.0, 16: 21 | 17.7;  2048 x 4096: 16: 10.2 | 13.1
-//   16-bit tokens, scales along K (uint4, groups of 128): 14336 x 4096: 8 tokens 19.1 | 30.8, 16: 25.7 | 31.8, 32:
+//   16-bit tokens, scales along K (uint4, groups of 128): 14336 x 4096: 8 tokens 18.4 | 30.8, 16: 22.8 | 31.8, 32:
 //     36.2 | 32.0;  4096 x 4096: 32: 10.2 | 19.1;  8192 x 4096: 24: 19.5 | 23.3;  1024 x 8192, 16: 12.5 | 22.4;  groups
 //     of 32: 4096 x 4096, 8: 9.0 | 19.9, 8192 x 8192, 24: 68 | 55
 //   f32 tokens (three planes): 14336 x 4096: 16: 40 | 120;  4096 x 4096: 24: 18.4 | 58;  4096 x 11008: 8: 19 | 82

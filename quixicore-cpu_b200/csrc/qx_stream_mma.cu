@@ -356,7 +356,9 @@ __global__ void __launch_bounds__(kThreads, CTAS) stream_scaled_kernel(const Sca
   constexpr int kBytes = kNibbles ? kColumns / 2 : kColumns;
   constexpr int kWords = kBytes / 4;
   constexpr int kFrags = kColumns / 8;
-  constexpr bool kEarly = PLANES == 1 && NT * kFrags <= 4;  // activations asked for one step ahead
+  // activations asked for one step ahead, where that spills nothing (two tiles of rows, uint4, 16 tokens on 14336 x 4096:
+  // 25.4 us with it, 22.8 without; one tile of rows, 4096 x 4096: 7.8 against 10.0)
+  constexpr bool kEarly = PLANES == 1 && MR == 1 && NT * kFrags <= 4;
   constexpr int kR = 16 * MR;
   constexpr int kPitch = 8 * NT + 1;
   __shared__ float red[kWarps][kR][kPitch];
@@ -821,8 +823,8 @@ qx_status launch(void (*kernel)(Params...), long long grid, int block, cudaStrea
 
 // Weight rows per warp: two tiles of 16 (every B fragment then feeds two MMAs) where that leaves more
 // than one CTA per SM, else one and more CTAs. Measured (us, two tiles | one): int8 digits of 4 tokens
-// 14336 x 4096 17.2 | 22.8, W8A8 24 rows 4096 x 4096 10.2 | 7.6; uint4, 4 tokens 14336 x 4096 19.1 | 20.1,
-// 4096 x 4096 9.2 | 6.3; 16 tokens 14336 x 4096 25.7 | 31.3.
+// 14336 x 4096 17.2 | 22.8, W8A8 24 rows 4096 x 4096 10.2 | 7.6; uint4, 8 tokens 14336 x 4096 18.4 | 20.1,
+// 4096 x 4096 9.2 | 6.3; 16 tokens 14336 x 4096 22.8 | 28.4.
 constexpr long long kWideRows = 32 * 192;
 
 int column_tiles(long long columns) { return columns <= 8 ? 1 : (columns <= 16 ? 2 : (columns <= 32 ? 4 : 8)); }
