@@ -11,7 +11,7 @@
 //
 // Both matmuls are weight-streaming kernels for decode-sized batches: a warp owns an output
 // channel, lanes read 16 bytes (32 weights) at a time, the weights are read ONCE for up to
-// MT activation rows; W4A8 batches go to the tensor cores instead (see "W4A8 on the tensor
+// MT activation rows; W4A8 batches go to MMAs instead (qx_stream_mma.cu, "W4A8 on the tensor
 // cores"). W4A8 multiplies with dp4a (the nibbles of a word as two unsigned
 // operands against the even / odd activation codes, the -8 folded into 8 * sum(codes) per
 // row) and reproduces the reference bit for bit: exact int32 dot, then
@@ -509,18 +509,10 @@ size_t tensor_scratch_bytes(long long m, long long k) {
   return align_up(rows * row_bytes, 256) + align_up(rows * 4, 256) + align_up(kTensorCounterBytes, 256) +
          tensor_piece_bytes(m);
 }
-// Where it is the faster one (us, here | dp4a kernel).
-// Rows on whole vectors: 512 x 2048: 16 rows 16.5 | 14.5, 24: 16.5 | 20.5;  2048 x 2048: 13: 16.0 | 15.0,
-// 16: 16.4 | 16.8;  1024 x 8192: 13: 30.7 | 39.8;  4096 x 4096: 12: 23.5 | 23.3, 13: 23.7 | 25.0, 64: 32 | 106;
-// 8192 x 4096: 8: 26.9 | 24.6;  14336 x 4096: 5: 34.0 | 30.8, 6: 34.8 | 34.8, 8: 35.7 | 42.9;
-// 28672 x 8192: 5: 89 | 93.
-// Rows that start anywhere: 512 x 2050: 2 rows 15.9 | 11.4, 4: 16.2 | 18.2;  1024 x 1030: 4: 13.5 | 12.6,
-// 8: 13.8 | 19.5;  4096 x 1026: 2: 15.2 | 19.3;  2048 x 4098: 1: 19.4 | 33.1;  4096 x 4098: 32: 26.5 | 581.
+// More rows than are streamed (below), where the dp4a kernel repeats the weights' work per row: 4096 x 4096, 64 rows 32 us
+// here against 106, 14336 x 4096, 8 rows 36 against 43.
 bool tensor_route(long long m, long long n, long long k) {
-  if (m > kTensorMaxRows || n < 128 || k > kTensorMaxK) return false;
-  const long long weights = n * k;
-  if (k % 32 != 0) return m >= 4 || (m >= 2 && weights >= (1LL << 22)) || weights >= (1LL << 23);
-  return m >= 17 || (m >= 13 && weights >= (1LL << 23)) || (m >= 5 && m * weights >= (5LL << 26));
+  return m > kStreamColumns && m <= kTensorMaxRows && n >= 128 && k <= kTensorMaxK;
 }
 qx_status launch_w4a8_tensor(const uint8_t* packed, const float* weight_scales, const float* x, float* y,
                              uint8_t* scratch, long long m, long long n, long long k, bool* served,

@@ -894,7 +894,7 @@ bool scaled_gemm_serves(const ScaledGemmArgs& a) {
   if (a.m < 1 || a.m > 65535 || a.rows < 1 || a.rows > (1LL << 26) || a.columns > (1LL << 24)) return false;
   // rows of codes and of activations start on 16 bytes, groups on a converter's 32 columns
   if (a.source == kScaledNibblesLoose) {  // (activations in rows of whole 16-byte vectors)
-    return a.group == a.columns && a.token_scales != nullptr && a.x_type == QX_STORAGE_F16 &&
+    return a.m > Small::kTokens && a.group == a.columns && a.token_scales != nullptr && a.x_type == QX_STORAGE_F16 &&
            a.x_stride % 8 == 0 && reinterpret_cast<uintptr_t>(a.codes) % 16 == 0;
   }
   const long long row_bytes = a.source == kScaledNibbles ? a.columns / 2 : a.columns;
@@ -981,9 +981,8 @@ qx_status launch_scaled_gemm(const ScaledGemmArgs& a, void* scratch, int* counte
   switch (a.source) {
     case kScaledNibbles:
       return launch_source<kScaledNibbles>(small, a.x_type, map_w, map_x, p, plan.grid, stream);
-    case kScaledNibblesLoose:  // (f16 activations only)
-      return small ? launch_kernel<kScaledNibblesLoose, false, 1, Small>(map_w, map_x, p, plan.grid, stream)
-                   : launch_kernel<kScaledNibblesLoose, false, 1, Large>(map_w, map_x, p, plan.grid, stream);
+    case kScaledNibblesLoose:  // (f16 activations, more tokens than a small tile has)
+      return launch_kernel<kScaledNibblesLoose, false, 1, Large>(map_w, map_x, p, plan.grid, stream);
     case kScaledBytes:
       return launch_source<kScaledBytes>(small, a.x_type, map_w, map_x, p, plan.grid, stream);
     default:  // (bf16 activations only)

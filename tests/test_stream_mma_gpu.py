@@ -99,3 +99,50 @@ def test_values_that_are_not_finite(qx, oracle_mod, layout, group):
         assert status == qx.OK and not np.isfinite(y[1]).any() and np.isnan(y[2]).all()
         status, want = weights.qgemm_storage(_storage(clean, x_type)[0], x_type, m)
         assert status == qx.OK and np.array_equal(y[[0, 3, 4]].view(np.uint32), want[[0, 3, 4]].view(np.uint32))
+
+
+# back to back on one scratch, with nothing waiting between: each call's activations take the place of those that the
+# call in front may still be reading, and the launches overlap
+@pytest.mark.parametrize("layout,group,m,x_type", [(INT8, 0, 3, BF16), (UINT4, 128, 12, F16), (UINT4, 128, 6, F32)])
+def test_chained_calls(qx, oracle_mod, layout, group, m, x_type):
+    import torch
+    n, k = 4096, 4096
+    rng = np.random.Generator(np.random.Philox(key=[9, group + m]))
+    weights, _ = _tensor(qx, oracle_mod, rng, layout, group, n, k)
+    types = {F32: torch.float32, F16: torch.float16, BF16: torch.bfloat16}
+    xs = [torch.randn((m, k), device="cuda").to(types[x_type]) for _ in range(3)]
+    want = []
+    for x in xs:
+        want.append(torch.zeros((m, n), device="cuda"))
+        assert weights.qgemm_storage_dev(x, x_type, want[-1], F32, m) == qx.OK, qx.last_error()
+        torch.cuda.synchronize()
+    got = [torch.zeros((m, n), device="cuda") for _ in range(60)]
+    torch.cuda.synchronize()
+    for i, y in enumerate(got):
+        assert weights.qgemm_storage_dev(xs[i % 3], x_type, y, F32, m) == qx.OK, qx.last_error()
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, want[i % 3]) for i, y in enumerate(got))
+
+
+def test_chained_w4a8(qx):
+    import torch
+    m, n, k = 16, 4096, 4096
+    w = torch.randint(0, 256, (n * k // 2,), dtype=torch.uint8, device="cuda")
+    ws = torch.rand(n, device="cuda") + 0.5
+    scratch = torch.zeros(int(qx.lib.qx_lowbit_w8a8_scratch_bytes(m, k)), dtype=torch.uint8, device="cuda")
+    xs = [torch.randn((m, k), device="cuda") for _ in range(3)]
+
+    def call(x, y):
+        assert qx.lib.qx_lowbit_gemm_w8a8_dev(w.data_ptr(), ws.data_ptr(), x.data_ptr(), y.data_ptr(), scratch.data_ptr(),
+                                              m, n, k, torch.cuda.current_stream().cuda_stream) == qx.OK, qx.last_error()
+
+    want = [torch.zeros((m, n), device="cuda") for _ in xs]
+    for x, y in zip(xs, want):
+        call(x, y)
+        torch.cuda.synchronize()
+    got = [torch.zeros((m, n), device="cuda") for _ in range(60)]
+    torch.cuda.synchronize()
+    for i, y in enumerate(got):
+        call(xs[i % 3], y)
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, want[i % 3]) for i, y in enumerate(got))
