@@ -18,7 +18,8 @@
 //
 // Measured (us, before | here): W4A8 16 rows 4096 x 4096 22.6 | 8.3; W8A8 4 rows 1024 x 1408 6.2 | 2.9; int8 1 token
 // 14336 x 4096 17.2 | 15.6 (3.8 TB/s); uint4 16 tokens 14336 x 4096 31.8 | 22.8 (1.4 TB/s). 16-bit activations are bound
-// by instruction issue at four warps per scheduler: a third of the instructions convert nibbles.
+// by the latency of loads at four warps per scheduler (more than half of the cycles between two instructions of a
+// warp), which the registers of 32 rows x 16 tokens leave no room to ask for earlier.
 //
 // tcgen05 would need both operands in shared memory and a TMEM round trip per scale group; at
 // these batch sizes the tensor work is a few percent of what either path could do.
