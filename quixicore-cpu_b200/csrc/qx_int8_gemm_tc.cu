@@ -159,7 +159,8 @@ struct __align__(16) TcBarriers {
 // accumulators (epilogue overlaps the next tile). NA = 2: 256 x bn outputs from one
 // activation slab per step -- a third less operand traffic from L2 per MAC, which is what
 // bounds this shape -- at the price of a single accumulator set (all 512 TMEM columns).
-template <int NA>
+// STAGES: the ring's slabs where they are as many as the largest tiles have (its steps are then constants), 0: p.stages.
+template <int NA, int STAGES>
 __global__ void __launch_bounds__(kThreads, 1) int8_gemm_tc_kernel(
     const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
     const TcParams p) {
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(kThreads, 1) int8_gemm_tc_kernel(
   const uint32_t a_bytes = NA * kBM * kBK;
   const uint32_t b_bytes = static_cast<uint32_t>(p.bn) * kBK;
   const uint32_t stage_bytes = a_bytes + b_bytes;
-  const uint32_t stages = static_cast<uint32_t>(p.stages);
+  const uint32_t stages = STAGES > 0 ? STAGES : static_cast<uint32_t>(p.stages);
   TcBarriers* bars = reinterpret_cast<TcBarriers*>(smem + stages * stage_bytes);
   float* as_tile = reinterpret_cast<float*>(bars + 1);  // [2][256] activation scales
   int* zp_tile = reinterpret_cast<int*>(as_tile + 2 * 256);
@@ -182,7 +183,7 @@ __global__ void __launch_bounds__(kThreads, 1) int8_gemm_tc_kernel(
   volatile int* abort_flag = &bars->abort_flag;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kMaxStages; ++s) {
+    for (uint32_t s = 0; s < stages; ++s) {
       mbar_init(&bars->full[s], 1);
       mbar_init(&bars->empty[s], 1);
     }
@@ -494,11 +495,11 @@ bool int8_gemm_tc_supported(const Int8GemmArgs& a) {
 }
 
 namespace {
-template <int NA>
-qx_status launch_tc_na(const CUtensorMap& map_w, const CUtensorMap& map_x, const TcParams& p,
+template <int NA, int STAGES>
+qx_status launch_tc_stages(const CUtensorMap& map_w, const CUtensorMap& map_x, const TcParams& p,
                        int grid, cudaStream_t stream) {
   static SmemOptIn opt_in;
-  QX_TRY(opt_in.ensure(int8_gemm_tc_kernel<NA>, kSmemMax));
+  QX_TRY(opt_in.ensure(int8_gemm_tc_kernel<NA, STAGES>, kSmemMax));
   cudaLaunchAttribute attribute{};
   attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute.val.programmaticStreamSerializationAllowed = 1;
@@ -509,9 +510,17 @@ qx_status launch_tc_na(const CUtensorMap& map_w, const CUtensorMap& map_x, const
   config.stream = stream;
   config.attrs = &attribute;
   config.numAttrs = 1;
-  QX_CUDA_TRY(cudaLaunchKernelEx(&config, int8_gemm_tc_kernel<NA>, map_w, map_x, p));
+  QX_CUDA_TRY(cudaLaunchKernelEx(&config, int8_gemm_tc_kernel<NA, STAGES>, map_w, map_x, p));
   count_launch();
   return QX_STATUS_OK;
+}
+
+template <int NA>
+qx_status launch_tc_na(const CUtensorMap& map_w, const CUtensorMap& map_x, const TcParams& p,
+                       int grid, cudaStream_t stream) {
+  constexpr int kLargest = NA == 2 ? 3 : 4;
+  return p.stages == kLargest ? launch_tc_stages<NA, kLargest>(map_w, map_x, p, grid, stream)
+                              : launch_tc_stages<NA, 0>(map_w, map_x, p, grid, stream);
 }
 
 // Scratch of the stream-K split, one per device, kept for the life of the process:
