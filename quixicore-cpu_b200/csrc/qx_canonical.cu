@@ -1141,13 +1141,16 @@ qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_t
   scaled.y_type = y_type;
   scaled.ldy = w->rows;
   if (stream_digits_route(w, m)) {
-    const size_t digit_bytes = align_up(stream_code_bytes(4 * m, w->columns), 256);
+    // (eight digits where the digit kernels below would give every 16 columns an envelope; qx_stream_mma.cu)
+    const int per_token = m < kPrefillTokens ? 8 : 4;
+    const size_t digit_bytes = align_up(stream_code_bytes(per_token * m, w->columns), 256);
     StreamIntArgs s{};
     s.source = kStreamBytes;
     s.result = kStreamDigits;
     s.prepared = true;
     s.codes = w->data;
-    s.x_rows = static_cast<int>(4 * m);
+    s.x_rows = static_cast<int>(per_token * m);
+    s.digits = per_token;
     s.rows = w->rows;
     s.columns = w->columns;
     s.ws = w->scales;
@@ -1162,7 +1165,7 @@ qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_t
       s.x = reinterpret_cast<const int8_t*>(scratch);
       s.as = reinterpret_cast<const float*>(scratch + digit_bytes);
       QX_TRY(launch_stream_digits(x, x_type, reinterpret_cast<int8_t*>(scratch),
-                                  reinterpret_cast<float*>(scratch + digit_bytes), m, w->columns, stream));
+                                  reinterpret_cast<float*>(scratch + digit_bytes), m, w->columns, per_token, stream));
       return launch_stream_int(s, stream);
     }
   }

@@ -27,7 +27,10 @@
 // Whole numbers (launch_stream_int): m16n8k32 s8 x s8 or u8 x s8 (nibbles as they are, the -8 of
 // the format through the activations' sums), int32 sums over the whole row. A canonical int8 tensor's
 // activations enter as four digit rows per token (31-bit fixed point under the token's envelope,
-// as canonical_row_digits_kernel has it), joined in 64-bit integers.
+// as canonical_row_digits_kernel has it), joined in 64-bit integers. Up to four tokens have eight: the digit kernel for
+// such batches gives every 16 columns an envelope of their own, and with one for the whole token an activation
+// 2^20 times the others would leave them ten bits (5.6e-4 of a result that does not see the large one). The second four
+// rows are the remainders under the remainders' envelope; they fill MMA columns that would be padding for one token.
 //
 // 16-bit activations (launch_stream_scaled): the arithmetic of qx_scaled_gemm.cu: whole numbers of
 // at most eight bits times f16 or bf16, sums of at most 128 columns (64 with three planes, 32 of
@@ -146,7 +149,7 @@ struct IntParams {
   int32_t* acc;
   long long row_bytes, x_stride, ldy;
   int rows, columns, x_rows, steps;
-  int result, activation, y_type, prepared;
+  int result, activation, y_type, prepared, digits;
 };
 
 // A step is 64 columns: 16 per lane of a quad (16 bytes of int8, 8 bytes of nibbles).
@@ -300,20 +303,25 @@ __global__ void __launch_bounds__(kThreads, CTAS) stream_int_kernel(const IntPar
     const int r = threadIdx.x % kR;
     const int row = row0 + r;
     if (p.result == kStreamDigits) {
-      const int c = threadIdx.x / kR;  // token of the two
-      const int token = 2 * n + c;
-      if (c < 2 && row < p.rows && 4 * token < p.x_rows) {
+      auto joined = [&](int first) {  // four digits
         long long total = 0;
 #pragma unroll
         for (int d = 3; d >= 0; --d) {
           int part = 0;
 #pragma unroll
-          for (int w = 0; w < kWarps; ++w) part += red[w][r][4 * c + d];
+          for (int w = 0; w < kWarps; ++w) part += red[w][r][first + d];
           total = total * 256 + part;
         }
+        return static_cast<double>(total);
+      };
+      const int tokens = 8 / p.digits;  // of these columns
+      const int c = threadIdx.x / kR, token = tokens * n + c;
+      if (c < tokens && row < p.rows && token * p.digits < p.x_rows) {
+        double total = joined(p.digits * c);
+        if (p.digits == 8) total += joined(4) * static_cast<double>(p.as[2 * token + 1]);
         // (a token that holds a value that is not finite has a NaN for its envelope)
-        float out = static_cast<float>(static_cast<double>(total) *
-                                       (static_cast<double>(p.as[token]) * static_cast<double>(__ldg(p.ws + row))));
+        const float e = p.as[p.digits == 8 ? 2 * token : token];
+        float out = static_cast<float>(total * (static_cast<double>(e) * static_cast<double>(__ldg(p.ws + row))));
         if (p.bias != nullptr) out += __ldg(p.bias + row);
         if (p.activation != QX_ACTIVATION_NONE) out = projection_activation(out, p.activation);
         store_output(p.y, p.y_type, token * p.ldy + row, out);
@@ -765,13 +773,37 @@ __global__ void __launch_bounds__(kRowThreads) stream_codes_kernel(const float* 
   }
 }
 
+// The whole number nearest to t, for any t below 2^31 (the conversion unit, at 16 a cycle, would bound the kernel).
+__device__ __forceinline__ float nearest_whole(float t) {
+  const float s = copysignf(8388608.0f, t);  // (2^23: from there on t has no fraction)
+  return fabsf(t) < 8388608.0f ? __fsub_rn(__fadd_rn(t, s), s) : t;
+}
+// The four balanced base-256 digits of each of four numbers, as four words of one digit each.
+__device__ __forceinline__ void digit_words(const int (&t)[4], uint32_t (&word)[4]) {
+  uint32_t v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = (static_cast<uint32_t>(t[i]) + 0x00808080u) ^ 0x00808080u;
+  const uint32_t low01 = __byte_perm(v[0], v[1], 0x5140), low23 = __byte_perm(v[2], v[3], 0x5140);
+  const uint32_t high01 = __byte_perm(v[0], v[1], 0x7362), high23 = __byte_perm(v[2], v[3], 0x7362);
+  word[0] = __byte_perm(low01, low23, 0x5410);
+  word[1] = __byte_perm(low01, low23, 0x7632);
+  word[2] = __byte_perm(high01, high23, 0x5410);
+  word[3] = __byte_perm(high01, high23, 0x7632);
+}
+
+// DIGITS rows per token: 4, or 8 with the remainders of the first four in the last. kDigitCtas CTAs per token: each takes
+// both maxima over the whole row and writes its share of the digits, so that no SM converts a row alone (one token, both
+// launches on 4096 x 4096, weights from memory: 8.2 us; 8.4 with one CTA and a shift and a mask per digit; four digits 7.4).
+constexpr int kDigitCtas = 4;
+template <int DIGITS>
 __global__ void __launch_bounds__(kRowThreads) stream_digits_kernel(const void* __restrict__ x, int x_type,
                                                                     int8_t* __restrict__ digits, float* __restrict__ e_out,
                                                                     long long columns, int column_tiles, int vector) {
   launch_dependents();  // (the projection's weights are prepared ones)
   wait_for_kernel_in_front();
-  __shared__ float warp_max[kRowThreads / 32];
-  const long long token = blockIdx.x, base = token * columns;
+  __shared__ float warp_max[kRowThreads / 32], warp_rest[kRowThreads / 32];
+  const long long token = blockIdx.x / kDigitCtas, base = token * columns;
+  const int share = blockIdx.x % kDigitCtas;
   const long long groups = (columns + 63) / 64 * 8;  // (whole steps)
   float held[kHeld][8];
   float amax = 0.0f;
@@ -783,30 +815,59 @@ __global__ void __launch_bounds__(kRowThreads) stream_digits_kernel(const void* 
     }
   });
   amax = block_max(amax, warp_max);
-  // envelope 2^E > amax, t = x * 2^30 / 2^E; tokens below 2^-70 altogether count as zero
-  int biased = static_cast<int>(__float_as_uint(amax) >> 23) + 1;
-  biased = biased < 58 ? 58 : biased;
+  // envelope 2^E > amax, t = x * 2^30 / 2^E; four digits: an activation below 2^-100 counts as zero
+  auto exponent = [](float maximum) {
+    const int biased = static_cast<int>(__float_as_uint(maximum) >> 23) + 1;
+    return biased < 58 ? 58 : biased;
+  };
+  auto fixed = [](int biased) { return __uint_as_float(static_cast<uint32_t>(284 - biased) << 23); };
+  const int biased = exponent(amax);
   const bool finite = biased < 256;
-  const float to_fixed = finite ? __uint_as_float(static_cast<uint32_t>(284 - biased) << 23) : 0.0f;
-  for_groups(x, x_type, base, columns, groups, vector != 0, held, false, [&](long long at, const float (&v)[8]) {
-    uint32_t word[4][2] = {};
+  const float to_fixed = finite ? fixed(biased) : 0.0f;
+  auto scaled = [&](float v) { return finite ? __fmul_rn(v, to_fixed) : 0.0f; };
+  int rest_biased = 58;
+  if (DIGITS == 8) {
+    float rmax = 0.0f;
+    for_groups(x, x_type, base, columns, groups, vector != 0, held, false, [&](long long, const float (&v)[8]) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      int rest = finite ? __float2int_rn(v[i] * to_fixed) : 0;
+      for (int i = 0; i < 8; ++i) {
+        const float t = scaled(v[i]);
+        rmax = fmaxf(rmax, fabsf(__fsub_rn(t, nearest_whole(t))));  // (exact)
+      }
+    });
+    rest_biased = exponent(block_max(rmax, warp_rest));
+  }
+  const float rest_fixed = fixed(rest_biased);
+  for_groups(x, x_type, base, columns, groups, vector != 0, held, false, [&](long long at, const float (&v)[8]) {
+    if ((at / 32) % kDigitCtas != share) return;  // (a warp's groups together)
+#pragma unroll
+    for (int half = 0; half < DIGITS / 4; ++half) {
+      uint32_t word[2][4];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        int whole[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float t = scaled(v[4 * q + i]);
+          whole[i] = __float2int_rn(half == 0 ? t : __fmul_rn(__fsub_rn(t, nearest_whole(t)), rest_fixed));
+        }
+        digit_words(whole, word[q]);
+      }
 #pragma unroll
       for (int d = 0; d < 4; ++d) {
-        const int digit = d < 3 ? ((rest + 128) & 255) - 128 : rest;
-        word[d][i >> 2] |= static_cast<uint32_t>(digit & 255) << (8 * (i & 3));
-        rest = (rest - digit) >> 8;
+        *reinterpret_cast<uint2*>(digits + fragment_byte(DIGITS * token + 4 * half + d, 8 * at, column_tiles)) =
+            make_uint2(word[0][d], word[1][d]);
       }
     }
-#pragma unroll
-    for (int d = 0; d < 4; ++d) {
-      *reinterpret_cast<uint2*>(digits + fragment_byte(4 * token + d, 8 * at, column_tiles)) = make_uint2(word[d][0], word[d][1]);
-    }
   });
-  if (threadIdx.x == 0) {
-    e_out[token] = finite ? __uint_as_float(static_cast<uint32_t>(biased - 30) << 23) : __uint_as_float(0x7fc00000u);
+  if (threadIdx.x == 0 && share == 0) {
+    const float e = finite ? __uint_as_float(static_cast<uint32_t>(biased - 30) << 23) : __uint_as_float(0x7fc00000u);
+    if (DIGITS == 8) {
+      e_out[2 * token] = e;
+      e_out[2 * token + 1] = __uint_as_float(static_cast<uint32_t>(rest_biased - 30) << 23);
+    } else {
+      e_out[token] = e;
+    }
   }
 }
 
@@ -938,6 +999,7 @@ qx_status launch_stream_int(const StreamIntArgs& a, cudaStream_t stream) {
   p.activation = a.activation;
   p.y_type = a.y_type;
   p.prepared = a.prepared ? 1 : 0;
+  p.digits = a.digits;
   switch (a.source) {
     case kStreamBytes:
       return a.result == kStreamDigits ? launch_int<kStreamBytes, true>(p, stream)
@@ -957,9 +1019,10 @@ qx_status launch_stream_codes(const float* x, int8_t* codes, float* scales, int*
                 (columns + 63) / 64 * 64, column_tiles(m), vector);
 }
 qx_status launch_stream_digits(const void* x, int x_type, int8_t* digits, float* e, long long m, long long columns,
-                               cudaStream_t stream) {
+                               int per_token, cudaStream_t stream) {
   const int vector = reinterpret_cast<uintptr_t>(x) % 16 == 0 ? 1 : 0;
-  return launch(stream_digits_kernel, m, kRowThreads, stream, x, x_type, digits, e, columns, column_tiles(4 * m), vector);
+  return launch(per_token == 8 ? stream_digits_kernel<8> : stream_digits_kernel<4>, kDigitCtas * m, kRowThreads, stream, x,
+                x_type, digits, e, columns, column_tiles(per_token * m), vector);
 }
 
 bool stream_scaled_serves(const StreamScaledArgs& a) {

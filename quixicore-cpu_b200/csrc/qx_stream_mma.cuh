@@ -12,14 +12,14 @@ enum StreamSource {
   kStreamNibblesLoose,  // the same, rows on any byte (int8 activations only)
 };
 
-constexpr int kStreamColumns = 64;  // activation rows (digit planes: four per token) at most
+constexpr int kStreamColumns = 64;  // activation rows (digit planes: four or eight per token) at most
 
 // ---- whole numbers on both sides (one weight scale per row) --------------------------------
 // What becomes of a row's exact int32 sums.
 enum StreamResult {
   kStreamW8A8,    // (sum - zp[t] * row_sum[o]) * ws[o] * as[t], two rounded multiplies
   kStreamW4A8,    // (sum - 8 * code_sums[t]) * ws[o] * as[t]
-  kStreamDigits,  // four digit rows per token: (sum_d 256^d * sum[d]) * (as[t] * ws[o]), bias, activation
+  kStreamDigits,  // four or eight digit rows per token: their sums joined, times e[t] * ws[o], bias, activation
 };
 struct StreamIntArgs {
   StreamSource source;
@@ -27,10 +27,11 @@ struct StreamIntArgs {
   const uint8_t* codes;
   const int8_t* x;        // W8A8: [x_rows][columns] int8, rows on 16 bytes; otherwise what the kernels below wrote
   int x_rows;
+  int digits;             // digits: rows per token, 4 or 8
   long long rows, columns;
   bool prepared;          // the codes are the library's: they may be read before the kernel in front is done
   const float* ws;        // [rows]
-  const float* as;        // [tokens]
+  const float* as;        // [tokens]; eight digits: [tokens][2]
   const int32_t* row_sum; // W8A8 with zero points: [rows], else null
   const int* zp;          // W8A8: [tokens]; W4A8: the code sums [tokens]
   const float* bias;      // digits: [rows] or null
@@ -48,10 +49,11 @@ qx_status launch_stream_int(const StreamIntArgs& a, cudaStream_t stream);
 size_t stream_code_bytes(long long x_rows, long long columns);
 qx_status launch_stream_codes(const float* x, int8_t* codes, float* scales, int* sums, long long m, long long columns,
                               cudaStream_t stream);
-// Digits: four rows per token (columns a multiple of 16) and the envelope: x = e * sum_d 256^d * digit_d
-// to 31 bits of the token's largest magnitude.
+// Digits (columns a multiple of 16). Four rows per token and the envelope: x = e * sum_d 256^d * digit_d to 31 bits of
+// the token's largest magnitude. Eight: what that leaves over has an envelope of its own, e[2t] * (the first four +
+// e[2t + 1] * the last four), so that a large activation takes no bits from the small ones beside it.
 qx_status launch_stream_digits(const void* x, int x_type, int8_t* digits, float* e, long long m, long long columns,
-                               cudaStream_t stream);
+                               int per_token, cudaStream_t stream);
 
 // ---- 16-bit activations, scales along K ------------------------------------------------------
 struct StreamScaledArgs {

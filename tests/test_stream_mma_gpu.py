@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from test_canonical_gpu import BF16, F16, F32, INT4, INT8, OUT_TOLERANCE, UINT4, activation_f64, close, widen
-from test_scaled_gemm_gpu import _product_f64, _storage, _tensor
+from test_scaled_gemm_gpu import CHANNEL, _product_f64, _storage, _tensor
 from test_w4a8_tensor_gpu import _exact
 
 pytestmark = pytest.mark.gpu
@@ -84,6 +84,32 @@ def test_canonical(qx, oracle_mod, layout, group, n, k, m, x_type):
     status, typed = weights.qgemm_storage(x, x_type, m, y_type=BF16, bias=bias, activation=3)
     assert status == qx.OK, qx.last_error()
     assert close(widen(typed, BF16), activation_f64(exact + bias.astype(np.float64)[None, :], 3), OUT_TOLERANCE[BF16])
+
+
+# An activation far above the others of its token, met by codes of zero in its 16 columns: the others keep the bits that
+# they have without it. 2^-24 of the result: one rounding each, and fixed-point steps of 2^-31 below the others. (A token of
+# size 1e35 gives results of up to 5e37; f32 ends at 3.4e38.)
+@pytest.mark.parametrize("m,x_type,size,outlier", [
+    (1, BF16, 1.0, 0.0), (1, BF16, 1.0, 2.0 ** 10), (4, BF16, 1.0, 2.0 ** 20), (1, F32, 1.0, 2.0 ** 26), (3, F32, 1.0, 2.0 ** 60),
+    (2, F16, 0.01, 2.0 ** 15), (1, BF16, 1e-25, 0.0), (4, F32, 1e-33, 0.0), (2, F32, 1e-20, 1e10), (1, F32, 1e35, 0.0)])
+def test_a_wide_range_within_a_token(qx, m, x_type, size, outlier):
+    n, k, column = 2048, 4096, 1000
+    rng = np.random.Generator(np.random.Philox(key=[n + m, int(outlier % 1000)]))
+    codes = rng.integers(-127, 128, (n, k), dtype=np.int8)
+    codes[:, column // 16 * 16:column // 16 * 16 + 16] = 0
+    scales = rng.uniform(0.002, 0.03, n).astype(np.float32)
+    weights = qx.CanonicalWeights()
+    view = qx.canonical_view(INT8, CHANNEL, n, k, k, codes.view(np.uint8).reshape(-1), scales)
+    assert weights.prepare(view) == qx.OK, qx.last_error()
+    values = (rng.standard_normal((m, k)) * size).astype(np.float32)
+    if outlier:
+        values[:, column] = outlier
+    x, x_exact = _storage(values, x_type)
+    exact = (x_exact.astype(np.float64) @ codes.astype(np.float64).T) * scales.astype(np.float64)
+    status, y = weights.qgemm_storage(x, x_type, m)
+    assert status == qx.OK, qx.last_error()
+    error = np.linalg.norm((y - exact) / size, axis=1) / np.linalg.norm(exact / size, axis=1)
+    assert np.all(error <= 2.0 ** -24), error
 
 
 @pytest.mark.parametrize("layout,group", [(INT8, 0), (UINT4, 128)])
