@@ -1053,7 +1053,9 @@ bool scaled_route(const qx_canonical_weights* w, int x_type, long long m) {
 // along K stay on the digit kernels, whose rows do not depend on the batch.
 constexpr long long kStreamWork = 1LL << 22;
 bool stream_digits_route(const qx_canonical_weights* w, long long m) {
-  return w->layout == QX_CANONICAL_INT8_SYMMETRIC && w->groups_per_row == 1 && m * w->rows * w->columns >= kStreamWork &&
+  // one to four tokens go the same way, whatever their number, so that a token's bits do not depend on it
+  const long long tokens = m < kPrefillTokens ? kPrefillTokens - 1 : m;
+  return w->layout == QX_CANONICAL_INT8_SYMMETRIC && w->groups_per_row == 1 && tokens * w->rows * w->columns >= kStreamWork &&
          (m <= 8 || (m <= kStreamColumns / 4 && m * w->rows <= (1LL << 16)));
 }
 bool stream_scaled_route(const qx_canonical_weights* w, int x_type, long long m) {
@@ -1159,7 +1161,7 @@ qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_t
     s.y = y;
     s.y_type = y_type;
     s.ldy = w->rows;
-    if (stream_int_serves(s) && digit_bytes + 256 <= kStreamScratchBytes) {
+    if (stream_int_serves(s) && (m < kPrefillTokens || digit_bytes + 256 <= kStreamScratchBytes)) {
       QX_TRY(workspace->reserve(kWorkspaceCounterBytes + digit_bytes + 256));
       uint8_t* scratch = static_cast<uint8_t*>(workspace->base) + kWorkspaceCounterBytes;
       s.x = reinterpret_cast<const int8_t*>(scratch);

@@ -112,6 +112,19 @@ def test_a_wide_range_within_a_token(qx, m, x_type, size, outlier):
     assert np.all(error <= 2.0 ** -24), error
 
 
+# below, at and above the line of the streamed route; rows whose digits outgrow the small scratch
+@pytest.mark.parametrize("n,k", [(256, 1024), (1023, 1024), (1024, 1024), (1500, 2048), (2048, 2048), (32, 40000)])
+def test_one_to_four_tokens_have_the_bits_of_one(qx, oracle_mod, n, k):
+    rng = np.random.Generator(np.random.Philox(key=[n, k]))
+    weights, _ = _tensor(qx, oracle_mod, rng, INT8, 0, n, k)
+    x, _ = _storage(rng.standard_normal((4, k)).astype(np.float32), BF16)
+    single = [weights.qgemm_storage(x[i:i + 1], BF16, 1)[1][0] for i in range(4)]
+    for m in (2, 3, 4):
+        status, y = weights.qgemm_storage(x[:m], BF16, m)
+        assert status == qx.OK, qx.last_error()
+        assert all(np.array_equal(y[i].view(np.uint32), single[i].view(np.uint32)) for i in range(m)), m
+
+
 @pytest.mark.parametrize("layout,group", [(INT8, 0), (UINT4, 128)])
 def test_values_that_are_not_finite(qx, oracle_mod, layout, group):
     n, k, m = 1000, 1024, 5
