@@ -289,8 +289,21 @@ __global__ void __launch_bounds__(kThreads, CTAS) stream_int_kernel(const IntPar
     }
   }
   // eight columns at a time: the warps' parts of K are added, exactly
+  const int r = threadIdx.x % kR;
+  const int row = row0 + r;
+  const bool eight = p.digits == 8;  // digits per token: one token of eight columns, or two
+  const int digit_at = threadIdx.x / kR;
 #pragma unroll
   for (int n = 0; n < NT; ++n) {
+    const int digit_token = eight ? n : 2 * n + digit_at;
+    const bool digit_mine = p.result == kStreamDigits && digit_at < (eight ? 1 : 2) && row < p.rows &&
+                            digit_token * (eight ? 8 : 4) < p.x_rows;
+    float digit_e = 0.0f, digit_rest = 0.0f, digit_ws = 0.0f;
+    if (digit_mine) {  // (asked for before the sums meet)
+      digit_e = p.as[eight ? 2 * digit_token : digit_token];
+      if (eight) digit_rest = p.as[2 * digit_token + 1];
+      digit_ws = __ldg(p.ws + row);
+    }
     if (n > 0) __syncthreads();
 #pragma unroll
     for (int i = 0; i < MR; ++i) {
@@ -300,31 +313,26 @@ __global__ void __launch_bounds__(kThreads, CTAS) stream_int_kernel(const IntPar
       }
     }
     __syncthreads();
-    const int r = threadIdx.x % kR;
-    const int row = row0 + r;
     if (p.result == kStreamDigits) {
-      auto joined = [&](int first) {  // four digits
-        long long total = 0;
+      if (digit_mine) {
+        auto joined = [&](int first) {  // four digits
+          long long total = 0;
 #pragma unroll
-        for (int d = 3; d >= 0; --d) {
-          int part = 0;
+          for (int d = 3; d >= 0; --d) {
+            int part = 0;
 #pragma unroll
-          for (int w = 0; w < kWarps; ++w) part += red[w][r][first + d];
-          total = total * 256 + part;
-        }
-        return static_cast<double>(total);
-      };
-      const int tokens = 8 / p.digits;  // of these columns
-      const int c = threadIdx.x / kR, token = tokens * n + c;
-      if (c < tokens && row < p.rows && token * p.digits < p.x_rows) {
-        double total = joined(p.digits * c);
-        if (p.digits == 8) total += joined(4) * static_cast<double>(p.as[2 * token + 1]);
+            for (int w = 0; w < kWarps; ++w) part += red[w][r][first + d];
+            total = total * 256 + part;
+          }
+          return static_cast<double>(total);
+        };
+        double total = joined(eight ? 0 : 4 * digit_at);
+        if (eight) total += joined(4) * static_cast<double>(digit_rest);
         // (a token that holds a value that is not finite has a NaN for its envelope)
-        const float e = p.as[p.digits == 8 ? 2 * token : token];
-        float out = static_cast<float>(total * (static_cast<double>(e) * static_cast<double>(__ldg(p.ws + row))));
+        float out = static_cast<float>(total * (static_cast<double>(digit_e) * static_cast<double>(digit_ws)));
         if (p.bias != nullptr) out += __ldg(p.bias + row);
         if (p.activation != QX_ACTIVATION_NONE) out = projection_activation(out, p.activation);
-        store_output(p.y, p.y_type, token * p.ldy + row, out);
+        store_output(p.y, p.y_type, digit_token * p.ldy + row, out);
       }
     } else {
       const int token = 8 * n + threadIdx.x / kR;
@@ -792,8 +800,9 @@ __device__ __forceinline__ void digit_words(const int (&t)[4], uint32_t (&word)[
 }
 
 // DIGITS rows per token: 4, or 8 with the remainders of the first four in the last. kDigitCtas CTAs per token: each takes
-// both maxima over the whole row and writes its share of the digits, so that no SM converts a row alone (one token, both
-// launches on 4096 x 4096, weights from memory: 8.2 us; 8.4 with one CTA and a shift and a mask per digit; four digits 7.4).
+// the maxima over the whole row and writes its share of the digits, so that no SM converts a row alone (one token, both
+// launches on 4096 x 4096, weights from memory: 7.6 us; 8.4 with one CTA, a shift and a mask per digit and the remainders'
+// maximum in every row; four digits 7.3).
 constexpr int kDigitCtas = 4;
 template <int DIGITS>
 __global__ void __launch_bounds__(kRowThreads) stream_digits_kernel(const void* __restrict__ x, int x_type,
@@ -801,20 +810,29 @@ __global__ void __launch_bounds__(kRowThreads) stream_digits_kernel(const void* 
                                                                     long long columns, int column_tiles, int vector) {
   launch_dependents();  // (the projection's weights are prepared ones)
   wait_for_kernel_in_front();
-  __shared__ float warp_max[kRowThreads / 32], warp_rest[kRowThreads / 32];
+  __shared__ float warp_max[kRowThreads / 32], warp_least[kRowThreads / 32], warp_rest[kRowThreads / 32];
   const long long token = blockIdx.x / kDigitCtas, base = token * columns;
   const int share = blockIdx.x % kDigitCtas;
   const long long groups = (columns + 63) / 64 * 8;  // (whole steps)
+  const float infinity = __uint_as_float(0x7f800000u);
   float held[kHeld][8];
-  float amax = 0.0f;
+  float amax = 0.0f, least = infinity;  // of the row; of the largest of any eight columns that are not all zero
   for_groups(x, x_type, base, columns, groups, vector != 0, held, true, [&](long long, const float (&v)[8]) {
+    float largest = 0.0f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {  // (fmaxf drops a NaN)
       const float a = fabsf(v[i]);
-      amax = a < __uint_as_float(0x7f800000u) ? fmaxf(amax, a) : __uint_as_float(0x7f800000u);
+      largest = a < infinity ? fmaxf(largest, a) : infinity;
     }
+    amax = fmaxf(amax, largest);
+    if (DIGITS == 8 && largest > 0.0f) least = fminf(least, largest);
   });
-  amax = block_max(amax, warp_max);
+  if (DIGITS == 8) {
+#pragma unroll
+    for (int h = 16; h >= 1; h >>= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, h));
+    if ((threadIdx.x & 31) == 0) warp_least[threadIdx.x >> 5] = least;
+  }
+  amax = block_max(amax, warp_max);  // (and its barrier)
   // envelope 2^E > amax, t = x * 2^30 / 2^E; four digits: an activation below 2^-100 counts as zero
   auto exponent = [](float maximum) {
     const int biased = static_cast<int>(__float_as_uint(maximum) >> 23) + 1;
@@ -825,17 +843,23 @@ __global__ void __launch_bounds__(kRowThreads) stream_digits_kernel(const void* 
   const bool finite = biased < 256;
   const float to_fixed = finite ? fixed(biased) : 0.0f;
   auto scaled = [&](float v) { return finite ? __fmul_rn(v, to_fixed) : 0.0f; };
-  int rest_biased = 58;
+  // A remainder is at most a half. Under that envelope eight columns keep the 23 bits that they would have under their
+  // own down to 2^-39 of the row's; a row with smaller ones beside its largest takes the largest remainder's envelope.
+  int rest_biased = 127;
   if (DIGITS == 8) {
-    float rmax = 0.0f;
-    for_groups(x, x_type, base, columns, groups, vector != 0, held, false, [&](long long, const float (&v)[8]) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float t = scaled(v[i]);
-        rmax = fmaxf(rmax, fabsf(__fsub_rn(t, nearest_whole(t))));  // (exact)
-      }
-    });
-    rest_biased = exponent(block_max(rmax, warp_rest));
+    for (int w = 0; w < kRowThreads / 32; ++w) least = fminf(least, warp_least[w]);
+    if (least < __uint_as_float(static_cast<uint32_t>(finite ? biased - 39 : 1) << 23)) {
+      float rmax = 0.0f;
+      for_groups(x, x_type, base, columns, groups, vector != 0, held, false, [&](long long, const float (&v)[8]) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float t = scaled(v[i]);
+          rmax = fmaxf(rmax, fabsf(__fsub_rn(t, nearest_whole(t))));  // (exact)
+        }
+      });
+      rest_biased = exponent(block_max(rmax, warp_rest));
+    }
   }
   const float rest_fixed = fixed(rest_biased);
   for_groups(x, x_type, base, columns, groups, vector != 0, held, false, [&](long long at, const float (&v)[8]) {
