@@ -1066,8 +1066,41 @@ bool stream_scaled_route(const qx_canonical_weights* w, int x_type, long long m)
   if (m > 16 && (m * w->rows > (1LL << 18) || (w->groups_per_row > 1 && w->group_size % 64 != 0))) return false;
   return x_type != QX_STORAGE_F32 || m * w->rows * w->columns >= (1LL << 25);
 }
-// Their scratch: no more than a workspace has that served the calls before (it grows by whole MiB, counters in front).
+// Their scratch, where one to four row-scaled tokens do not set it: what the first MiB of a workspace holds behind the
+// counters.
 constexpr size_t kStreamScratchBytes = (1 << 20) - 4096;
+
+// The most scratch that the routes for small batches take for any call of at most m tokens, whatever its activations' type
+// and alignment. Every call reserves it, so that a workspace that has served a batch does not grow for a smaller
+// one (which would free what captured calls point into, and cannot be done during a capture). `prefill_from`: the
+// number of tokens from which int8 with one scale per row takes the digit planes.
+size_t small_batch_bytes(const qx_canonical_weights* w, bool digits, long long prefill_from, long long m) {
+  if (!digits) return 0;
+  const bool planes = w->layout == QX_CANONICAL_INT8_SYMMETRIC && w->groups_per_row == 1;
+  const bool prefill = planes && w->columns <= 131000;
+  size_t bytes = digit_image_bytes(prefill && m >= prefill_from ? prefill_from - 1 : m, w->columns);
+  auto at_least = [&](size_t more) { bytes = more > bytes ? more : bytes; };
+  if (planes) {
+    const long long few = m < kPrefillTokens ? m : kPrefillTokens - 1;
+    at_least(align_up(stream_code_bytes(8 * few, w->columns), 256) + 256);
+    if (m >= kPrefillTokens) {
+      const long long rows = 4 * (m < kStreamColumns / 4 ? m : kStreamColumns / 4);
+      const size_t more = align_up(stream_code_bytes(rows, w->columns), 256) + 256;
+      at_least(more < kStreamScratchBytes ? more : kStreamScratchBytes);
+    }
+    if (prefill && m >= prefill_from) at_least(prefill_scratch_bytes(m, w->rows, w->columns));
+  } else if (m >= 5) {
+    StreamScaledArgs s{};
+    s.source = w->layout == QX_CANONICAL_INT8_SYMMETRIC ? kStreamBytes : kStreamNibbles;
+    s.columns = w->columns;
+    s.group = w->groups_per_row == 1 ? w->columns : w->group_size;
+    s.x_type = QX_STORAGE_F32;
+    s.m = m < 32 ? m : 32;
+    const size_t more = stream_scaled_scratch_bytes(s);
+    at_least(more < kStreamScratchBytes ? more : kStreamScratchBytes);
+  }
+  return bytes;
+}
 
 qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_type,
                            const float* bias, void* y, int y_type, long long m, int activation,
@@ -1121,8 +1154,6 @@ qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_t
     if (asked > 0) prefill_from = asked;
   }
   const bool prefill = int8 && p.groups_per_row == 1 && m >= prefill_from && w->columns <= 131000;
-  const size_t image_bytes = prefill ? prefill_scratch_bytes(m, w->rows, w->columns)
-                                     : (digits ? digit_image_bytes(m, w->columns) : 0);
   // batches on the tensor cores with the scales applied per group (qx_scaled_gemm.cu)
   ScaledGemmArgs scaled{};
   scaled.source = int8 ? kScaledBytes : kScaledNibbles;
@@ -1142,6 +1173,16 @@ qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_t
   scaled.y = y;
   scaled.y_type = y_type;
   scaled.ldy = w->rows;
+  const int sm_count = ctx->prop.multiProcessorCount;
+  size_t least_bytes = gather_bytes + small_batch_bytes(w, digits, prefill_from, m);
+  // (as for the types that stream: a batch of the other type may be one for the tensor cores)
+  if ((scaled_route(w, QX_STORAGE_F16, m) || scaled_route(w, QX_STORAGE_F32, m)) && scaled_gemm_serves(scaled)) {
+    const size_t scaled_bytes = scaled_gemm_scratch_bytes(scaled, sm_count);
+    least_bytes = scaled_bytes > least_bytes ? scaled_bytes : least_bytes;
+  }
+  auto reserve = [&](size_t bytes) {
+    return workspace->reserve(kWorkspaceCounterBytes + (bytes > least_bytes ? bytes : least_bytes));
+  };
   if (stream_digits_route(w, m)) {
     // (eight digits where the digit kernels below would give every 16 columns an envelope; qx_stream_mma.cu)
     const int per_token = m < kPrefillTokens ? 8 : 4;
@@ -1162,7 +1203,7 @@ qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_t
     s.y_type = y_type;
     s.ldy = w->rows;
     if (stream_int_serves(s) && (m < kPrefillTokens || digit_bytes + 256 <= kStreamScratchBytes)) {
-      QX_TRY(workspace->reserve(kWorkspaceCounterBytes + digit_bytes + 256));
+      QX_TRY(reserve(digit_bytes + 256));
       uint8_t* scratch = static_cast<uint8_t*>(workspace->base) + kWorkspaceCounterBytes;
       s.x = reinterpret_cast<const int8_t*>(scratch);
       s.as = reinterpret_cast<const float*>(scratch + digit_bytes);
@@ -1192,29 +1233,24 @@ qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_t
     s.ldy = w->rows;
     const size_t stream_bytes = stream_scaled_scratch_bytes(s);
     if (stream_scaled_serves(s) && stream_bytes <= kStreamScratchBytes) {
-      if (stream_bytes != 0) QX_TRY(workspace->reserve(kWorkspaceCounterBytes + stream_bytes));
+      QX_TRY(reserve(stream_bytes));
       return launch_stream_scaled(s, stream_bytes != 0 ? static_cast<uint8_t*>(workspace->base) + kWorkspaceCounterBytes : nullptr,
                                   stream);
     }
   }
   if (scaled_route(w, x_type, m) && scaled_gemm_serves(scaled)) {
-    const int sm_count = ctx->prop.multiProcessorCount;
-    // (and what the digit kernels of smaller batches use)
-    const size_t scaled_bytes = scaled_gemm_scratch_bytes(scaled, sm_count);
-    QX_TRY(workspace->reserve(kWorkspaceCounterBytes + (scaled_bytes > gather_bytes + image_bytes
-                                                            ? scaled_bytes
-                                                            : gather_bytes + image_bytes)));
+    QX_TRY(reserve(0));
     return launch_scaled_gemm(scaled, static_cast<uint8_t*>(workspace->base) + kWorkspaceCounterBytes,
                               static_cast<int*>(workspace->base), kWorkspaceCounterBytes, sm_count,
                               ctx->error_dev, stream);
   }
   uint32_t* image = nullptr;
-  if (gather_bytes + image_bytes != 0) {
-    QX_TRY(workspace->reserve(kWorkspaceCounterBytes + gather_bytes + image_bytes));
+  if (least_bytes != 0) {
+    QX_TRY(reserve(0));
     uint8_t* scratch = static_cast<uint8_t*>(workspace->base) + kWorkspaceCounterBytes;
     image = reinterpret_cast<uint32_t*>(scratch + gather_bytes);
     if (prefill) {
-      return launch_prefill_int8(p, scratch + gather_bytes, ctx->prop.multiProcessorCount, stream);
+      return launch_prefill_int8(p, scratch + gather_bytes, sm_count, stream);
     }
     if (w->act_order != nullptr) {
       float* gathered = reinterpret_cast<float*>(scratch);
@@ -1229,7 +1265,6 @@ qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_t
   }
   const int x_vector = p.x_type == QX_STORAGE_F32 ? 16 : 8;
   p.vector_x = (w->columns % 4 == 0 && reinterpret_cast<uintptr_t>(p.x) % x_vector == 0) ? 1 : 0;
-  const int sm_count = ctx->prop.multiProcessorCount;
   switch (w->layout) {
     case QX_CANONICAL_INT8_SYMMETRIC:
       return launch_any<QX_CANONICAL_INT8_SYMMETRIC>(p, digits, image, sm_count, stream);

@@ -77,6 +77,47 @@ def test_smaller_canonical_batches_are_captured(qx, oracle_mod, act_order):
     workspace.close()
 
 
+# Batches that stream their codes, on a workspace of their own: smaller ones of any type, off 16 bytes as well, take digit
+# images, digit planes, laid-out activations or the tensor cores
+@pytest.mark.parametrize("layout,group,n,k,order,m,x_type,smaller", [
+    (UINT4, 128, 4736, 1024, False, 8, BF16, [(8, F32), (5, F16), (4, BF16), (1, F32)]),
+    (UINT4, 128, 4736, 1024, False, 16, F16, [(16, F32), (9, BF16), (8, F16), (4, F32)]),
+    (INT4, 32, 4096, 2048, True, 6, F16, [(6, F32), (4, BF16), (1, F32)]),
+    (INT4, 128, 64, 40960, True, 5, BF16, [(5, F32), (4, F32), (1, F16)]),
+    (UINT4, 128, 8192, 8192, False, 32, F16, [(32, F32), (25, F32), (24, F32), (16, BF16), (1, F32)]),
+    (INT8, 0, 16384, 32, False, 8, BF16, [(7, F32), (5, BF16), (4, F32), (1, F16)]),
+    (INT8, 0, 4096, 4096, False, 16, BF16, [(12, F32), (8, F16), (5, BF16), (4, F32), (1, BF16)]),
+    (INT8, 0, 32, 40000, False, 4, F32, [(3, F32), (1, BF16)]),
+])
+def test_smaller_batches_of_a_streamed_one_are_captured(qx, oracle_mod, layout, group, n, k, order, m, x_type, smaller):
+    import torch
+    rng = np.random.Generator(np.random.Philox(key=[n + m, k]))
+    weights, _ = _tensor(qx, oracle_mod, rng, layout, group, n, k,
+                         act_order=rng.permutation(k).astype(np.int32) if order else None)
+    workspace = Workspace(qx)
+    x = torch.randn((m, k), device="cuda").to(getattr(torch, TORCH[x_type]))
+    y = torch.zeros((m, n), device="cuda")
+    assert canonical_call(qx, weights, x, x_type, y, workspace) == qx.OK, qx.last_error()
+    torch.cuda.synchronize()
+    capacity = workspace.capacity()
+    calls = []
+    for rows, kind in smaller:
+        for offset in (0, 1):
+            buffer = torch.zeros(rows * k + 1, device="cuda", dtype=getattr(torch, TORCH[kind]))
+            xs = buffer[offset:offset + rows * k].view(rows, k)
+            xs.copy_(torch.randn((rows, k), device="cuda"))
+            want = torch.zeros((rows, n), device="cuda")
+            assert canonical_call(qx, weights, xs, kind, want, workspace) == qx.OK, qx.last_error()
+            torch.cuda.synchronize()
+            assert workspace.capacity() == capacity, (rows, kind, offset)
+            calls.append((xs, kind, want))
+    for xs, kind, want in calls:  # (nothing has grown: now inside a capture)
+        got = torch.zeros_like(want)
+        captured(qx, lambda: canonical_call(qx, weights, xs, kind, got, workspace))
+        assert workspace.capacity() == capacity and torch.equal(got, want)
+    workspace.close()
+
+
 def test_smaller_q8_0_prompts_are_captured(qx, wl):
     import torch
     n, k = 4736, 1024
