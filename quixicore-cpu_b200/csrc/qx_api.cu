@@ -54,32 +54,45 @@ __global__ void __launch_bounds__(256) stage_in_kernel(const uint4* __restrict__
   const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < n16) dst[i] = src[i];
 }
-// The address at which the GPU reaches host memory that is pinned or registered, else null.
-void* device_address(const void* host) {
+// What the runtime knows about a caller's buffer. `device`: the address at which the GPU reaches host memory that is
+// pinned or registered, else null. `pageable`: host memory that the runtime does not know; all else (device or managed
+// memory, which the copies below take as well) is not for the CPU to touch.
+struct CallerMemory {
+  void* device = nullptr;
+  bool pageable = false;
+};
+CallerMemory caller_memory(const void* p) {
+  CallerMemory out;
   cudaPointerAttributes attributes{};
-  if (cudaPointerGetAttributes(&attributes, host) == cudaSuccess && attributes.type == cudaMemoryTypeHost) {
-    return attributes.devicePointer;
+  if (cudaPointerGetAttributes(&attributes, p) != cudaSuccess) {
+    (void)cudaGetLastError();  // unregistered host memory is not an error here
+    out.pageable = true;
+  } else if (attributes.type == cudaMemoryTypeHost) {
+    out.device = attributes.devicePointer;
+  } else {
+    out.pageable = attributes.type == cudaMemoryTypeUnregistered;
   }
-  (void)cudaGetLastError();  // unregistered host memory is not an error here
-  return nullptr;
+  return out;
 }
 // Small inputs in pageable memory take the same way through the context's pinned memory (its mutex is
 // held, and the call before has waited for its kernels).
 qx_status stage_in(DeviceContext* ctx, void* dst, const void* src, size_t bytes) {
   const cudaStream_t s = ctx->stream;
   if (bytes > 0 && bytes <= kBounceBytes && bytes % 16 == 0 && reinterpret_cast<uintptr_t>(dst) % 16 == 0) {
-    const void* from = reinterpret_cast<uintptr_t>(src) % 16 == 0 ? device_address(src) : nullptr;
-    if (from == nullptr) {
-      QX_TRY(ctx->ensure_bounce());
+    const CallerMemory memory = caller_memory(src);
+    const void* from = reinterpret_cast<uintptr_t>(src) % 16 == 0 ? memory.device : nullptr;
+    if (from == nullptr && (memory.pageable || memory.device != nullptr) && ctx->ensure_bounce() == QX_STATUS_OK) {
       std::memcpy(ctx->bounce_host, src, bytes);
       from = ctx->bounce_dev;
     }
-    const size_t n16 = bytes / 16;
-    stage_in_kernel<<<static_cast<unsigned>((n16 + 255) / 256), 256, 0, s>>>(static_cast<const uint4*>(from),
-                                                                              static_cast<uint4*>(dst), n16);
-    count_launch();
-    QX_CUDA_TRY(cudaGetLastError());
-    return QX_STATUS_OK;
+    if (from != nullptr) {
+      const size_t n16 = bytes / 16;
+      stage_in_kernel<<<static_cast<unsigned>((n16 + 255) / 256), 256, 0, s>>>(static_cast<const uint4*>(from),
+                                                                                static_cast<uint4*>(dst), n16);
+      count_launch();
+      QX_CUDA_TRY(cudaGetLastError());
+      return QX_STATUS_OK;
+    }
   }
   return h2d(dst, src, bytes, s);
 }
@@ -455,10 +468,11 @@ qx_status qx_qgemm_prepacked(const qx_weights* weights, const float* x, float* y
   // registered host memory): the kernel's row finishers write it over PCIe and the copy
   // back is saved. Small ones in pageable memory go to the context's pinned memory that way and
   // from there by the CPU; larger ones take the staged copy.
-  float* y_target = static_cast<float*>(device_address(y));
-  const bool direct = y_target != nullptr, bounced = !direct && y_bytes <= kBounceBytes;
+  const CallerMemory memory = caller_memory(y);
+  float* y_target = static_cast<float*>(memory.device);
+  const bool direct = y_target != nullptr;
+  const bool bounced = memory.pageable && y_bytes <= kBounceBytes && ctx->ensure_bounce() == QX_STATUS_OK;
   if (bounced) {
-    QX_TRY(ctx->ensure_bounce());
     y_target = reinterpret_cast<float*>(ctx->bounce_dev + kBounceBytes);
   } else if (!direct) {
     y_target = reinterpret_cast<float*>(st.at(off_y));

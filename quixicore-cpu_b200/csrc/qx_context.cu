@@ -46,11 +46,14 @@ qx_status DeviceContext::ensure_bounce() {
   if (bounce_host != nullptr) return QX_STATUS_OK;
   void* host = nullptr;
   void* dev = nullptr;
-  QX_CUDA_TRY(cudaHostAlloc(&host, 2 * kBounceBytes, cudaHostAllocMapped));
-  const cudaError_t mapped = cudaHostGetDevicePointer(&dev, host, 0);
-  if (mapped != cudaSuccess) {
-    (void)cudaFreeHost(host);
-    QX_CUDA_TRY(mapped);
+  cudaError_t code = cudaHostAlloc(&host, 2 * kBounceBytes, cudaHostAllocMapped);
+  if (code == cudaSuccess) {
+    code = cudaHostGetDevicePointer(&dev, host, 0);
+    if (code != cudaSuccess) (void)cudaFreeHost(host);
+  }
+  if (code != cudaSuccess) {  // (the caller copies instead)
+    (void)cudaGetLastError();
+    return QX_STATUS_OUT_OF_MEMORY;
   }
   bounce_host = static_cast<uint8_t*>(host);
   bounce_dev = static_cast<uint8_t*>(dev);
