@@ -1148,10 +1148,15 @@ qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_t
       w->act_order != nullptr ? align_up(static_cast<size_t>(m) * w->columns * sizeof(float), 256) : 0;
   // int8 with one scale per row, five tokens or more: the tensor-core route
   long long prefill_from = kPrefillTokens;
-  // developer switch: QX_B200_CANONICAL_PREFILL_TOKENS=<n> moves the threshold
+  // developer switches: QX_B200_CANONICAL_PREFILL_TOKENS=<n> moves the threshold, and from there on nothing streams; nor
+  // where the digit planes are to take the CUDA-core GEMM
+  bool planes_asked = int8_gemm_forced_simple();
   if (const char* forced = std::getenv("QX_B200_CANONICAL_PREFILL_TOKENS")) {
     const long long asked = std::atoll(forced);
-    if (asked > 0) prefill_from = asked;
+    if (asked > 0) {
+      prefill_from = asked;
+      planes_asked = true;
+    }
   }
   const bool prefill = int8 && p.groups_per_row == 1 && m >= prefill_from && w->columns <= 131000;
   // batches on the tensor cores with the scales applied per group (qx_scaled_gemm.cu)
@@ -1183,7 +1188,7 @@ qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_t
   auto reserve = [&](size_t bytes) {
     return workspace->reserve(kWorkspaceCounterBytes + (bytes > least_bytes ? bytes : least_bytes));
   };
-  if (stream_digits_route(w, m)) {
+  if (stream_digits_route(w, m) && !(prefill && planes_asked)) {
     // (eight digits where the digit kernels below would give every 16 columns an envelope; qx_stream_mma.cu)
     const int per_token = m < kPrefillTokens ? 8 : 4;
     const size_t digit_bytes = align_up(stream_code_bytes(per_token * m, w->columns), 256);

@@ -11,18 +11,17 @@
 #include "qx_stream_mma.cuh"
 
 namespace qx {
-namespace {
-bool force_simple() {
+
+bool int8_gemm_forced_simple() {
   static const bool forced = []() {
     const char* v = std::getenv("QX_B200_INT8_GEMM_VARIANT");
     return v != nullptr && std::strcmp(v, "dp4a") == 0;
   }();
   return forced;
 }
-}  // namespace
 
 const char* int8_gemm_variant_name() {
-  return force_simple() ? "sm100a_dp4a" : "sm100a_tcgen05_i8";
+  return int8_gemm_forced_simple() ? "sm100a_dp4a" : "sm100a_tcgen05_i8";
 }
 
 namespace {
@@ -53,8 +52,8 @@ bool stream_route(const Int8GemmArgs& a, StreamIntArgs* s) {
 
 qx_status launch_int8_gemm(const Int8GemmArgs& a, cudaStream_t stream) {
   StreamIntArgs s{};
-  if (!force_simple() && stream_route(a, &s)) return launch_stream_int(s, stream);
-  if (!force_simple() && int8_gemm_tc_supported(a)) return launch_int8_gemm_tc(a, stream);
+  if (!int8_gemm_forced_simple() && stream_route(a, &s)) return launch_stream_int(s, stream);
+  if (!int8_gemm_forced_simple() && int8_gemm_tc_supported(a)) return launch_int8_gemm_tc(a, stream);
   return launch_int8_gemm_simple(a, stream);
 }
 

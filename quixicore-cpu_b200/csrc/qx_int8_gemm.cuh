@@ -52,5 +52,7 @@ qx_status launch_int4_offset8_digits(const uint8_t* packed, const float* scales,
                                      long long groups, long long group_size, cudaStream_t stream);
 
 const char* int8_gemm_variant_name();
+// whether QX_B200_INT8_GEMM_VARIANT=dp4a asks for the CUDA-core kernel
+bool int8_gemm_forced_simple();
 
 }  // namespace qx
