@@ -495,19 +495,16 @@ constexpr size_t kTensorCounterBytes = scaled_gemm_counter_bytes(kTensorCtas);
 long long code_stride(long long k) { return (k + 7) / 8 * 8; }
 // tiles of more tokens are not cut into pieces (there are enough of them)
 constexpr long long kTensorPieceTokens = 128;
-size_t tensor_piece_bytes(long long m) {
-  const long long tokens = m <= 64 ? (m + 31) / 32 * 32 : kTensorPieceTokens;
-  return static_cast<size_t>(kTensorCtas) * 2 * 128 * tokens * sizeof(float);
-}
+constexpr size_t kTensorPieceBytes = static_cast<size_t>(kTensorCtas) * 2 * 128 * kTensorPieceTokens * sizeof(float);
 constexpr long long kTensorMaxRows = 65535;
-// What any call of at most `m` rows and `k` columns uses: a scratch of one size serves all smaller
+// What any call of at most `m` rows and `k` columns uses there: a scratch of one size serves all smaller
 // calls, so the pieces are counted where this call would have none, and the rows and columns up to
 // the limits of the tensor route.
 size_t tensor_scratch_bytes(long long m, long long k) {
   const size_t rows = static_cast<size_t>(m < kTensorMaxRows ? m : kTensorMaxRows);
   const size_t row_bytes = static_cast<size_t>(code_stride(k < kTensorMaxK ? k : kTensorMaxK)) * 2;
   return align_up(rows * row_bytes, 256) + align_up(rows * 4, 256) + align_up(kTensorCounterBytes, 256) +
-         tensor_piece_bytes(m);
+         kTensorPieceBytes;
 }
 // More rows than are streamed (below), where the dp4a kernel repeats the weights' work per row: 4096 x 4096, 64 rows 32 us
 // here against 106, 14336 x 4096, 8 rows 36 against 43.
@@ -558,6 +555,9 @@ qx_status launch_w4a8_tensor(const uint8_t* packed, const float* weight_scales, 
 // 32: 12.6 | 25.7;  14336 x 8190: 8: 37.6 | 72.9, 40: 67.5 | 76.7;  4096 x 8190: 64: 29 | 42.6.
 bool stream_route(long long m, long long k) { return m <= kStreamColumns && (m > 2 || k % 32 != 0); }
 // Small batches: codes streamed past the activations (qx_stream_mma.cu). Scratch: [codes][scales][sums].
+size_t stream_scratch_bytes(long long m, long long k) {
+  return align_up(stream_code_bytes(m, k), 256) + 2 * align_up(static_cast<size_t>(m) * 4, 256);
+}
 qx_status launch_w4a8_stream(const uint8_t* packed, const float* weight_scales, const float* x, float* y,
                              uint8_t* scratch, long long m, long long n, long long k, bool* served,
                              cudaStream_t stream) {
@@ -692,13 +692,15 @@ qx_status qx_quantize_int8(const float* x, int8_t* codes, float* scales, long lo
 }
 
 // lowbit_gemm_w8a8 on the device: x f32 [m][k]; scratch_dev holds the activation codes,
-// scales and code sums, or those in 16 bits with counters and pieces of tiles:
-// qx_lowbit_w8a8_scratch_bytes(m, k) bytes, never fewer for more rows or columns.
+// scales and code sums (in rows, or in the order of the streamed products' lanes), or those in 16 bits with counters and
+// pieces of tiles: qx_lowbit_w8a8_scratch_bytes(m, k) bytes, the most that a call of at most m rows and k columns uses.
 size_t qx_lowbit_w8a8_scratch_bytes(long long m, long long k) {
   if (m <= 0 || k <= 0) return 0;
   const size_t codes = align_up(static_cast<size_t>(m) * k, 256) + 2 * align_up(static_cast<size_t>(m) * 4, 256);
-  const size_t tensor = tensor_scratch_bytes(m, k);
-  return codes > tensor ? codes : tensor;
+  const size_t stream = stream_scratch_bytes(m < kStreamColumns ? m : kStreamColumns, k);
+  const size_t tensor = m > kStreamColumns ? tensor_scratch_bytes(m, k) : 0;
+  const size_t most = codes > stream ? codes : stream;
+  return most > tensor ? most : tensor;
 }
 
 qx_status qx_lowbit_gemm_w8a8_dev(const uint8_t* packed_dev, const float* weight_scales_dev,
