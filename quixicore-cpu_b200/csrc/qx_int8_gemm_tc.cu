@@ -36,6 +36,7 @@
 #include <mutex>
 
 #include "qx_int8_gemm.cuh"
+#include "qx_int8_tiles.h"
 #include "qx_sm100.cuh"
 
 namespace qx {
@@ -570,41 +571,10 @@ bool choose_stream_k(long long tiles128, int k_slabs, int sm_count) {
   return tiles128 * k_slabs >= sm_count && tiles128 <= kStreamKMaxTiles;
 }
 
-// A tile's channels (na tiles of 128) and tokens: the pair for which the slowest SM is done first. Cycles of a
-// 32-byte step of K: what shared memory has to take in and give out at 128 bytes a cycle, (na * 128 + bn) rows
-// fetched and na * (128 + bn) read, above the tensor pipe's na * bn / 2 for every tile; and no less than the 100 at which a
-// ring of small slabs still hides the fetches. The results of an SM's last tile are stored with nothing beside them.
-// Measured (us, chosen here | 256 tokens and 256 channels wherever they gave six of ten SMs a tile): 200 rows 2048 x 8192
-// 15.2 | 30.9, 512 rows 1024 x 4096 7.0 | 13.7, 128 rows 4096 x 4096 7.7 | 11.6, 300 rows 14336 x 4096 26.4 | 37.4, 1300 rows
-// 9000 x 2048 29.2 | 41.3, 2048 rows 1024 x 1024 5.1 | 7.2; 512 rows 14336 x 4096 30.0 either way.
-struct TileChoice {
-  int na, bn;
-};
-TileChoice choose_tile(long long m, long long n, long long k, int sm_count) {
-  int forced_na = 0;
-  if (const char* forced = std::getenv("QX_B200_INT8_WEIGHT_TILES")) {
-    if (forced[0] == '1' || forced[0] == '2') forced_na = forced[0] - '0';
-  }
-  const long long steps = (k + 31) / 32;
-  TileChoice best{1, 32};
-  long long best_cycles = -1;
-  for (int na = 1; na <= 2; ++na) {
-    if (forced_na != 0 && na != forced_na) continue;
-    for (int bn = 256; bn >= 32; bn -= 32) {
-      if (bn > 32 && bn - 32 >= m) continue;  // (nothing but padding in the last 32)
-      const long long tiles = (n + na * kBM - 1) / (na * kBM) * ((m + bn - 1) / bn);
-      const long long rounds = (tiles + sm_count - 1) / sm_count;
-      const long long moved = (na * 128 + bn + na * (128 + bn)) / 4;
-      const long long cycles = rounds * steps * (moved > 100 ? moved : 100) + 6LL * na * bn;
-      // (smaller tiles for a tenth at least: their padding costs power, which large products are short of; 1024 rows
-      // 14336 x 4096 61 us with 224 tiles of 256 tokens, 63 with 280 of 224)
-      if (best_cycles < 0 || cycles * 10 < best_cycles * 9) {
-        best_cycles = cycles;
-        best = TileChoice{na, bn};
-      }
-    }
-  }
-  return best;
+// developer switch: QX_B200_INT8_WEIGHT_TILES=1|2 leaves tiles of 128 or 256 channels
+int forced_weight_tiles() {
+  const char* forced = std::getenv("QX_B200_INT8_WEIGHT_TILES");
+  return forced != nullptr && (forced[0] == '1' || forced[0] == '2') ? forced[0] - '0' : 0;
 }
 }  // namespace
 
@@ -620,7 +590,7 @@ qx_status launch_int8_gemm_tc(const Int8GemmArgs& a, cudaStream_t stream) {
                         choose_stream_k((a.n + kBM - 1) / kBM * r_tiles, k_slabs, sm_count);
   int na = 1;
   if (!stream_k) {
-    const TileChoice tile = choose_tile(a.m, a.n, a.k, sm_count);
+    const Int8Tile tile = choose_int8_tile(a.m, a.n, a.k, sm_count, forced_weight_tiles());
     na = tile.na;
     bn = tile.bn;
     r_tiles = (a.m + bn - 1) / bn;
