@@ -114,6 +114,11 @@ __device__ __forceinline__ uint4 load_activations(const uint8_t* src) {
 
 // Calls a CTA's rows of codes into L2. Before the wait for the kernel in front this reads nothing
 // on the program's behalf: should that kernel write these bytes, the lines in L2 change with them.
+// Only where the matrix is not much more than the CTAs of one round ask for at once: from there on the requests stand in the
+// way of the loads (us, with it | without: int8 16 rows 2048 x 2048 4.6 | 5.1, 4096 x 4096 7.6 | 8.0; 8192 x 4096
+// 10.5 | 10.2, 14336 x 8192 36 | 31, one token 28672 x 8192 68 | 54; uint4 16 tokens 8192 x 4096 13.5 | 12.8,
+// 14336 x 4096 24.2 | 23.2, 28672 x 8192 88 | 78; f32 tokens 4096 x 4096 14.1 | 14.9).
+constexpr long long kIntPrefetchBytes = (1LL << 25) - 1, kScaledPrefetchBytes = 1LL << 24;
 __device__ __forceinline__ void prefetch_rows(const uint8_t* codes, long long row_bytes, long long row0, int rows,
                                               long long total_rows) {
   const long long last = row0 + rows < total_rows ? row0 + rows : total_rows;
@@ -149,7 +154,7 @@ struct IntParams {
   int32_t* acc;
   long long row_bytes, x_stride, ldy;
   int rows, columns, x_rows, steps;
-  int result, activation, y_type, prepared, digits;
+  int prefetch, result, activation, y_type, prepared, digits;
 };
 
 // A step is 64 columns: 16 per lane of a quad (16 bytes of int8, 8 bytes of nibbles).
@@ -164,7 +169,7 @@ __global__ void __launch_bounds__(kThreads, CTAS) stream_int_kernel(const IntPar
   const int g = lane >> 2, t = lane & 3;
   const int row0 = blockIdx.x * kR;
   launch_dependents();
-  prefetch_rows(p.codes, p.row_bytes, row0, kR, p.rows);
+  if (p.prefetch != 0) prefetch_rows(p.codes, p.row_bytes, row0, kR, p.rows);
 
   // (offsets from the CTA's first row: a pointer per row would be two registers)
   const uint8_t* codes = p.codes + row0 * p.row_bytes + t * (kNibbles ? 8 : 16);
@@ -366,7 +371,7 @@ struct ScaledParams {
   long long row_bytes, x_stride, ldy;
   uint32_t nibble_xor;
   int rows, columns, m, steps, group, groups, flush_steps;
-  int activation, y_type;
+  int prefetch, activation, y_type;
 };
 
 // A step is 64 columns, or 32 where sums of 32 leave the tensor core: a quarter per lane of a quad.
@@ -387,7 +392,7 @@ __global__ void __launch_bounds__(kThreads, CTAS) stream_scaled_kernel(const Sca
   const int g = lane >> 2, t = lane & 3;
   const int row0 = blockIdx.x * kR;
   launch_dependents();
-  prefetch_rows(p.codes, p.row_bytes, row0, kR, p.rows);
+  if (p.prefetch != 0) prefetch_rows(p.codes, p.row_bytes, row0, kR, p.rows);
 
   // (offsets from the CTA's first row: a pointer per row would be two registers)
   const uint8_t* codes = p.codes + row0 * p.row_bytes + t * kBytes;
@@ -1023,6 +1028,7 @@ qx_status launch_stream_int(const StreamIntArgs& a, cudaStream_t stream) {
   p.activation = a.activation;
   p.y_type = a.y_type;
   p.prepared = a.prepared ? 1 : 0;
+  p.prefetch = p.row_bytes * a.rows <= kIntPrefetchBytes ? 1 : 0;
   p.digits = a.digits;
   switch (a.source) {
     case kStreamBytes:
@@ -1091,6 +1097,7 @@ qx_status launch_stream_scaled(const StreamScaledArgs& a, void* scratch, cudaStr
   p.activation = a.activation;
   p.y_type = a.y_type;
   p.flush_steps = promote_columns(a) / step;
+  p.prefetch = p.row_bytes * a.rows <= kScaledPrefetchBytes ? 1 : 0;
   const bool bf16 = a.x_type != QX_STORAGE_F16;
   return a.source == kStreamBytes ? launch_scaled<kStreamBytes>(p, bf16, planes, step, fragments, stream)
                                   : launch_scaled<kStreamNibbles>(p, bf16, planes, step, fragments, stream);
