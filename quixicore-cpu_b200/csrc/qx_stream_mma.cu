@@ -916,11 +916,15 @@ qx_status launch(void (*kernel)(Params...), long long grid, int block, cudaStrea
   return QX_STATUS_OK;
 }
 
-// Weight rows per warp: two tiles of 16 (every B fragment then feeds two MMAs) where that leaves more
-// than one CTA per SM, else one and more CTAs. Measured (us, two tiles | one): int8 digits of 4 tokens
-// 14336 x 4096 17.2 | 22.8, W8A8 24 rows 4096 x 4096 10.2 | 7.6; uint4, 8 tokens 14336 x 4096 18.4 | 20.1,
-// 4096 x 4096 9.2 | 6.3; 16 tokens 14336 x 4096 22.8 | 28.4.
-constexpr long long kWideRows = 32 * 192;
+// Weight rows per warp: two tiles of 16 (every B fragment then feeds two MMAs) where CTAs of one tile would be more than
+// two per SM, the third of which finds the SM full; one tile and more CTAs below that. Measured (us, two tiles | one): 8192 x
+// 4096: int8 digits of 4 tokens 13.0 | 18.7, W8A8 16 rows 10.5 | 14.6, uint4 8 tokens 10.7 | 13.2;  5120 x 5120: digits of 2
+// tokens 11.8 | 17.0, W8A8 16 rows 11.2 | 16.2, uint4 8 tokens 12.2 | 14.3, 16 tokens 14.3 | 16.6, W4A8 32 rows 14.4 | 20.7;
+// 4096 x 4096: uint4 8 tokens 9.2 | 6.3, W8A8 24 rows 10.2 | 7.6.
+constexpr long long kWideRows = 2 * 148 * 16 + 1;
+// One column tile of whole numbers has registers for three CTAs, and nibbles with two tiles one round more of them: digits of
+// one token 5120 x 5120 10.5 | 9.0, W4A8 16 rows 11.7 | 10.8.
+constexpr long long kWideRowsOfFew = 32 * 192;
 
 int column_tiles(long long columns) { return columns <= 8 ? 1 : (columns <= 16 ? 2 : (columns <= 32 ? 4 : 8)); }
 
@@ -929,7 +933,8 @@ qx_status launch_int(const IntParams& p, cudaStream_t stream) {
   constexpr bool kLoose = SRC == kStreamNibblesLoose;
   // (eight column tiles: one CTA per SM either way, and rows on any byte have no registers for two tiles of
   // rows: 40 tokens on 14336 x 8190 68 us against 91)
-  if (NT == 8 ? !kLoose : p.rows >= kWideRows) {
+  constexpr long long kWide = NT == 1 || (NT == 2 && SRC != kStreamBytes) ? kWideRowsOfFew : kWideRows;
+  if (NT == 8 ? !kLoose : p.rows >= kWide) {
     constexpr int kNT = NT == 8 && kLoose ? 4 : NT;
     return launch(stream_int_kernel<SRC, FRAGMENTS, kNT, 2, (NT <= 2 && SRC == kStreamNibbles ? 4 : 2), (NT == 8 ? 1 : 2)>,
                   (p.rows + 31) / 32, kThreads, stream, p);
