@@ -1041,30 +1041,45 @@ bool scaled_route(const qx_canonical_weights* w, int x_type, long long m) {
   return m >= (f32 ? 25 : 5) && m * w->rows * w->columns >= least;
 }
 
-// Which small batches stream the codes past their activations (qx_stream_mma.cu). Measured there | before (us):
-//   int8, one scale per row (four digit rows per token, exact sums): 14336 x 4096: 1 token 15.6 | 17.2, 4: 17.2 | 34.2,
-//     8: 20.6 | 20.7 (and one launch less);  4096 x 4096: 1: 6.0 | 6.8, 8: 8.2 | 12.6, 12: 9.9 | 15.2;  8192 x 4096:
-//     8: 10.9 | 17.0, 16: 21 | 17.7;  2048 x 4096: 16: 10.2 | 13.1
-//   16-bit tokens, scales along K (uint4, groups of 128): 14336 x 4096: 8 tokens 18.4 | 30.8, 16: 22.8 | 31.8, 32:
-//     36.2 | 32.0;  4096 x 4096: 32: 10.2 | 19.1;  8192 x 4096: 24: 19.5 | 23.3;  1024 x 8192, 16: 12.5 | 22.4;  groups
-//     of 32: 4096 x 4096, 8: 9.0 | 19.9, 8192 x 8192, 24: 68 | 55
-//   f32 tokens (three planes): 14336 x 4096: 16: 40 | 120;  4096 x 4096: 24: 18.4 | 58;  4096 x 11008: 8: 19 | 82
+// Which small batches stream the codes past their activations (qx_stream_mma.cu). Measured in graph replay, there | on the
+// other route (us):
+//   int8, one scale per row (exact sums, eight digit rows per token up to four tokens, then four; other route: digit kernel
+//   up to four tokens, then digit planes through the W8A8 GEMM):
+//     1 token: 1024 x 1024 3.6 | 3.7, 4096 x 4096 7.2 | 9.3, 14336 x 4096 16.8 | 17.3, 28672 x 8192 54 | 55;
+//     4: 4096 x 4096 9.5 | 16.9, 14336 x 4096 22.9 | 34.5, 28672 x 8192 68 | 115
+//     5: 5120 x 5120 13.1 | 16.1, 8192 x 4096 12.0 | 15.5, 14336 x 4096 21.2 | 19.0;  8: 4096 x 11008 20.1 | 22.3,
+//     8192 x 4096 12.8 | 13.8, 11008 x 4096 20.5 | 15.8, 28672 x 8192 66 | 50
+//     9: 4096 x 4096 11.7 | 13.9, 6144 x 4096 20.5 | 14.8;  15: 4096 x 8192 20.7 | 20.8;  16: 4096 x 4096 13.1 | 13.0,
+//     2048 x 8192 18.8 | 17.4, 4096 x 11008 25.0 | 22.8
+//   16-bit tokens, scales along K (uint4, groups of 128; other route: qx_scaled_gemm.cu): 14336 x 4096: 8 tokens 18.7 | 31.2,
+//     16: 23.2 | 32.2, 17: 36.8 | 32.6;  4096 x 4096: 32: 10.8 | 19.9;  5120 x 5120: 17: 23.6 | 22.7;  8192 x 4096: 32:
+//     20.3 | 24.3;  28672 x 8192: 16: 78 | 93;  4096 x 14336: 32: 31.7 | 34.8;  groups of 32: 11008 x 4096, 16: 37 | 45
+//   f32 tokens (three planes; other route: the digit kernels up to 24 tokens): 14336 x 4096: 16: 42 | 121;  4096 x 4096:
+//     24: 21.4 | 59, 32: 22.1 | 25.9;  5120 x 5120: 24: 42 | 85, 32: 42 | 29;  1024 x 2048: 17: 11.3 | 10.5, 32: 11.5 | 18.5
 // Not the smallest products, which are launches and nothing else on either route; and up to four tokens with scales
 // along K stay on the digit kernels, whose rows do not depend on the batch.
 constexpr long long kStreamWork = 1LL << 22;
 bool stream_digits_route(const qx_canonical_weights* w, long long m) {
+  if (w->layout != QX_CANONICAL_INT8_SYMMETRIC || w->groups_per_row != 1) return false;
   // one to four tokens go the same way, whatever their number, so that a token's bits do not depend on it
-  const long long tokens = m < kPrefillTokens ? kPrefillTokens - 1 : m;
-  return w->layout == QX_CANONICAL_INT8_SYMMETRIC && w->groups_per_row == 1 && tokens * w->rows * w->columns >= kStreamWork &&
-         (m <= 8 || (m <= kStreamColumns / 4 && m * w->rows <= (1LL << 16)));
+  if (m < kPrefillTokens) return (kPrefillTokens - 1) * w->rows * w->columns >= kStreamWork;
+  if (m * w->rows * w->columns < kStreamWork || w->columns > 16384) return false;
+  if (m <= 8) return w->rows <= 8192;
+  return w->rows <= 4096 && (m < 16 || (m == 16 && w->columns <= 4096));
 }
 bool stream_scaled_route(const qx_canonical_weights* w, int x_type, long long m) {
-  if (w->group_index != nullptr || !w->scales_have_room || m < 5 || m * w->rows * w->columns < kStreamWork) return false;
+  if (w->group_index != nullptr || !w->scales_have_room || m < 5 || m > 32 || m * w->rows * w->columns < kStreamWork) return false;
   // fractional zero points have no exact 16-bit form; int8 with one scale per row has exact sums above
   if (w->layout == QX_CANONICAL_UINT4_AFFINE && !w->integral_zeros) return false;
   if (w->layout == QX_CANONICAL_INT8_SYMMETRIC && w->groups_per_row == 1) return false;
-  if (m > 16 && (m * w->rows > (1LL << 18) || (w->groups_per_row > 1 && w->group_size % 64 != 0))) return false;
-  return x_type != QX_STORAGE_F32 || m * w->rows * w->columns >= (1LL << 25);
+  if (m > 16 && w->groups_per_row > 1 && w->group_size % 64 != 0) return false;
+  const bool f32 = x_type == QX_STORAGE_F32;
+  if (f32 && m * w->rows * w->columns < (m <= 16 ? 2LL << 24 : 3LL << 24)) return false;
+  if (m <= 16) return true;
+  // (CTAs of 16 rows, two per SM: one round of them, or where a second one is not nearly empty)
+  const bool one_round = w->rows <= 2 * 148 * 16;
+  if (f32) return one_round || (m <= 24 && m * w->rows <= (1LL << 18));
+  return one_round || (w->rows >= 6144 && w->rows <= 8192);
 }
 // Their scratch, where one to four row-scaled tokens do not set it: what the first MiB of a workspace holds behind the
 // counters.

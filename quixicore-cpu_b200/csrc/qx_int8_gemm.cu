@@ -25,12 +25,22 @@ const char* int8_gemm_variant_name() {
 }
 
 namespace {
-// Batches that qx_stream_mma.cu takes: few rows, where a tile of 128 or 256 channels leaves most SMs idle
-// (us, there | tensor-core kernel): 1024 x 1408, 4 rows 2.9 | 6.2;  4096 x 4096: 1: 5.5 | 8.7, 16: 6.2 | 9.2,
-// 24: 7.6 | 9.4;  8192 x 4096: 16: 8.0 | 14.3, 24: 11.3 | 14.9;  14336 x 4096: 4: 14.9 | 16.5, 16: 16.9 | 17.1,
-// 32: 23 | 15.4;  4096 x 8192: 32: 13.5 | 23.6;  4096 x 4096: 64: 10.6 | 9.0.
+// Batches that qx_stream_mma.cu takes: few rows on few channels, where tiles of 128 channels leave most SMs idle. With more
+// channels they do not, and the TMA rings of the tensor-core kernel read faster than the streamed loads; of longer rows the
+// warps' loads spread over more of them. Measured in graph replay (us, there | tensor-core kernel):
+//   1 row:   1024 x 1408 3.1 | 5.9;  4096 x 4096 7.5 | 9.8;  8192 x 4096 9.1 | 11.6;  4096 x 11008 15.4 | 18.3;
+//     11008 x 4096 15.0 | 14.2;  14336 x 8192 27.7 | 25.3;  28672 x 8192 52.5 | 46.6;  8192 x 28672 49.6 | 48.1
+//   16 rows: 4096 x 4096 7.6 | 10.2;  5120 x 5120 10.5 | 11.7;  8192 x 4096 10.2 | 11.9;  14336 x 4096 17.8 | 14.5;
+//     8192 x 28672 52 | 49
+//   24 rows: 4096 x 4096 8.8 | 10.4;  2048 x 8192 13.4 | 14.5;  4096 x 11008 18.5 | 18.9;  4096 x 28672 41.9 | 40.6;
+//     5120 x 5120 15.2 | 11.7
+//   32 rows, a whole tile of tokens there: 1024 x 1408 4.6 | 4.1;  4096 x 4096 9.2 | 8.1
+bool few_rows(const Int8GemmArgs& a) {
+  if (a.n <= 4096 && a.m <= kStreamW8A8Rows) return a.m <= 16 || a.k <= 16384;
+  return a.n <= 8192 && a.m <= 16 && a.k <= 16384;
+}
 bool stream_route(const Int8GemmArgs& a, StreamIntArgs* s) {
-  if (a.m > 32 || (a.m > 8 && a.m * a.n > (1LL << 18))) return false;
+  if (!few_rows(a)) return false;
   s->source = kStreamBytes;
   s->result = kStreamW8A8;
   s->codes = reinterpret_cast<const uint8_t*>(a.w);

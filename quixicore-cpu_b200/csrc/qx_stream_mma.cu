@@ -931,25 +931,30 @@ int column_tiles(long long columns) { return columns <= 8 ? 1 : (columns <= 16 ?
 
 template <StreamSource SRC, bool FRAGMENTS, int NT>
 qx_status launch_int(const IntParams& p, cudaStream_t stream) {
-  constexpr bool kLoose = SRC == kStreamNibblesLoose;
-  // (eight column tiles: one CTA per SM either way, and rows on any byte have no registers for two tiles of
-  // rows: 40 tokens on 14336 x 8190 68 us against 91)
+  // Eight column tiles: one CTA per SM either way, and rows on any byte have no registers for two tiles of
+  // rows (40 tokens on 14336 x 8190 68 us against 91). Four of W8A8 come with up to 4096 rows only.
+  constexpr bool kOne = SRC == kStreamNibblesLoose ? NT == 8 : (SRC == kStreamBytes && !FRAGMENTS && NT == 4);
+  constexpr bool kTwo = NT == 8 && SRC != kStreamNibblesLoose;
   constexpr long long kWide = NT == 1 || (NT == 2 && SRC != kStreamBytes) ? kWideRowsOfFew : kWideRows;
-  if (NT == 8 ? !kLoose : p.rows >= kWide) {
-    constexpr int kNT = NT == 8 && kLoose ? 4 : NT;
-    return launch(stream_int_kernel<SRC, FRAGMENTS, kNT, 2, (NT <= 2 && SRC == kStreamNibbles ? 4 : 2), (NT == 8 ? 1 : 2)>,
-                  (p.rows + 31) / 32, kThreads, stream, p);
+  if constexpr (!kOne) {
+    if (kTwo || p.rows >= kWide) {
+      return launch(stream_int_kernel<SRC, FRAGMENTS, NT, 2, (NT <= 2 && SRC == kStreamNibbles ? 4 : 2), (NT == 8 ? 1 : 2)>,
+                    (p.rows + 31) / 32, kThreads, stream, p);
+    }
   }
-  return launch(stream_int_kernel<SRC, FRAGMENTS, NT, 1, (NT == 8 ? 2 : 4), (NT == 8 ? 1 : (NT == 1 ? 3 : 2))>,
-                (p.rows + 15) / 16, kThreads, stream, p);
+  if constexpr (!kTwo) {
+    return launch(stream_int_kernel<SRC, FRAGMENTS, NT, 1, (NT == 8 ? 2 : 4), (NT == 8 ? 1 : (NT == 1 ? 3 : 2))>,
+                  (p.rows + 15) / 16, kThreads, stream, p);
+  }
 }
 template <StreamSource SRC, bool FRAGMENTS>
 qx_status launch_int(const IntParams& p, cudaStream_t stream) {
+  static_assert(kStreamW8A8Rows <= 32);
   switch (column_tiles(p.x_rows)) {
     case 1: return launch_int<SRC, FRAGMENTS, 1>(p, stream);
     case 2: return launch_int<SRC, FRAGMENTS, 2>(p, stream);
     case 4: return launch_int<SRC, FRAGMENTS, 4>(p, stream);
-    default: return launch_int<SRC, FRAGMENTS, 8>(p, stream);
+    default: return launch_int<SRC, FRAGMENTS, SRC == kStreamBytes && !FRAGMENTS ? 4 : 8>(p, stream);
   }
 }
 
@@ -1005,7 +1010,7 @@ bool wants_fragments(const StreamScaledArgs& a) {
 }  // namespace
 
 bool stream_int_serves(const StreamIntArgs& a) {
-  if (a.x_rows < 1 || a.x_rows > kStreamColumns || a.rows < 1 || a.rows > (1LL << 30) || a.columns > 131000) return false;
+  if (a.x_rows < 1 || a.x_rows > (a.result == kStreamW8A8 ? kStreamW8A8Rows : kStreamColumns) || a.rows < 1 || a.rows > (1LL << 30) || a.columns > 131000) return false;
   if (reinterpret_cast<uintptr_t>(a.x) % 16 != 0) return false;
   if (a.source == kStreamBytes) return a.columns % 16 == 0 && reinterpret_cast<uintptr_t>(a.codes) % 16 == 0;
   return a.source == kStreamNibblesLoose || (a.columns % 16 == 0 && reinterpret_cast<uintptr_t>(a.codes) % 8 == 0);
