@@ -155,7 +155,7 @@ struct IntParams {
   int32_t* acc;
   long long row_bytes, x_stride, ldy;
   int rows, columns, x_rows, steps;
-  int prefetch, result, activation, y_type, prepared, digits;
+  int prefetch, activation, y_type, prepared, digits;
 };
 
 // A step is 64 columns: 16 per lane of a quad (16 bytes of int8, 8 bytes of nibbles).
@@ -165,6 +165,8 @@ __global__ void __launch_bounds__(kThreads, CTAS) stream_int_kernel(const IntPar
   constexpr bool kNibbles = SRC != kStreamBytes;
   constexpr int kWords = SRC == kStreamNibbles ? 2 : 4;  // loose: the 16 bytes around a row's 8
   constexpr int kR = 16 * MR;
+  // (what becomes of the sums goes with the source: digits lie in the lanes' order beside bytes, W8A8 activations as they are)
+  constexpr bool kDigits = SRC == kStreamBytes && FRAGMENTS;
   __shared__ int red[kWarps][kR][9];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
@@ -297,12 +299,13 @@ __global__ void __launch_bounds__(kThreads, CTAS) stream_int_kernel(const IntPar
   // eight columns at a time: the warps' parts of K are added, exactly
   const int r = threadIdx.x % kR;
   const int row = row0 + r;
-  const bool eight = p.digits == 8;  // digits per token: one token of eight columns, or two
+  // Digits per token: one token of eight columns, or two. One and two tokens have eight, nine and more four.
+  const bool eight = NT <= 2 || (NT == 4 && p.digits == 8);
   const int digit_at = threadIdx.x / kR;
 #pragma unroll
   for (int n = 0; n < NT; ++n) {
     const int digit_token = eight ? n : 2 * n + digit_at;
-    const bool digit_mine = p.result == kStreamDigits && digit_at < (eight ? 1 : 2) && row < p.rows &&
+    const bool digit_mine = kDigits && digit_at < (eight ? 1 : 2) && row < p.rows &&
                             digit_token * (eight ? 8 : 4) < p.x_rows;
     float digit_e = 0.0f, digit_rest = 0.0f, digit_ws = 0.0f;
     if (digit_mine) {  // (asked for before the sums meet)
@@ -319,7 +322,7 @@ __global__ void __launch_bounds__(kThreads, CTAS) stream_int_kernel(const IntPar
       }
     }
     __syncthreads();
-    if (p.result == kStreamDigits) {
+    if constexpr (kDigits) {
       if (digit_mine) {
         auto joined = [&](int first) {  // four digits
           long long total = 0;
@@ -347,7 +350,7 @@ __global__ void __launch_bounds__(kThreads, CTAS) stream_int_kernel(const IntPar
 #pragma unroll
         for (int w = 0; w < kWarps; ++w) total += red[w][r][token & 7];
         float value;
-        if (p.result == kStreamW4A8) {
+        if constexpr (kNibbles) {
           value = static_cast<float>(total - 8 * p.zp[token]);
         } else {
           long long dot = total;
@@ -805,11 +808,10 @@ __device__ __forceinline__ void digit_words(const int (&t)[4], uint32_t (&word)[
   word[3] = __byte_perm(high01, high23, 0x7632);
 }
 
-// DIGITS rows per token: 4, or 8 with the remainders of the first four in the last. kDigitCtas CTAs per token: each takes
+// DIGITS rows per token: 4, or 8 with the remainders of the first four in the last. digit_ctas() CTAs per token: each takes
 // the maxima over the whole row and writes its share of the digits, so that no SM converts a row alone (one token, both
-// launches on 4096 x 4096, weights from memory: 7.6 us; 8.4 with one CTA, a shift and a mask per digit and the remainders'
-// maximum in every row; four digits 7.3).
-constexpr int kDigitCtas = 4;
+// launches on 4096 x 4096, weights from memory: 7.0 us with four; 16 tokens 11.6 with two, 11.8 with four).
+constexpr int digit_ctas(int digits) { return digits == 8 ? 4 : 2; }
 template <int DIGITS>
 __global__ void __launch_bounds__(kRowThreads) stream_digits_kernel(const void* __restrict__ x, int x_type,
                                                                     int8_t* __restrict__ digits, float* __restrict__ e_out,
@@ -817,6 +819,7 @@ __global__ void __launch_bounds__(kRowThreads) stream_digits_kernel(const void* 
   launch_dependents();  // (the projection's weights are prepared ones)
   wait_for_kernel_in_front();
   __shared__ float warp_max[kRowThreads / 32], warp_least[kRowThreads / 32], warp_rest[kRowThreads / 32];
+  constexpr int kDigitCtas = digit_ctas(DIGITS);
   const long long token = blockIdx.x / kDigitCtas, base = token * columns;
   const int share = blockIdx.x % kDigitCtas;
   const long long groups = (columns + 63) / 64 * 8;  // (whole steps)
@@ -1010,7 +1013,8 @@ bool wants_fragments(const StreamScaledArgs& a) {
 }  // namespace
 
 bool stream_int_serves(const StreamIntArgs& a) {
-  if (a.x_rows < 1 || a.x_rows > (a.result == kStreamW8A8 ? kStreamW8A8Rows : kStreamColumns) || a.rows < 1 || a.rows > (1LL << 30) || a.columns > 131000) return false;
+  const int most = a.result == kStreamW8A8 ? kStreamW8A8Rows : kStreamColumns;
+  if (a.x_rows < 1 || a.x_rows > most || a.rows < 1 || a.rows > (1LL << 30) || a.columns > 131000) return false;
   if (reinterpret_cast<uintptr_t>(a.x) % 16 != 0) return false;
   if (a.source == kStreamBytes) return a.columns % 16 == 0 && reinterpret_cast<uintptr_t>(a.codes) % 16 == 0;
   return a.source == kStreamNibblesLoose || (a.columns % 16 == 0 && reinterpret_cast<uintptr_t>(a.codes) % 8 == 0);
@@ -1035,7 +1039,6 @@ qx_status launch_stream_int(const StreamIntArgs& a, cudaStream_t stream) {
   p.columns = static_cast<int>(a.columns);
   p.x_rows = a.x_rows;
   p.steps = static_cast<int>((a.columns + 63) / 64);
-  p.result = a.result;
   p.activation = a.activation;
   p.y_type = a.y_type;
   p.prepared = a.prepared ? 1 : 0;
@@ -1062,8 +1065,8 @@ qx_status launch_stream_codes(const float* x, int8_t* codes, float* scales, int*
 qx_status launch_stream_digits(const void* x, int x_type, int8_t* digits, float* e, long long m, long long columns,
                                int per_token, cudaStream_t stream) {
   const int vector = reinterpret_cast<uintptr_t>(x) % 16 == 0 ? 1 : 0;
-  return launch(per_token == 8 ? stream_digits_kernel<8> : stream_digits_kernel<4>, kDigitCtas * m, kRowThreads, stream, x,
-                x_type, digits, e, columns, column_tiles(per_token * m), vector);
+  return launch(per_token == 8 ? stream_digits_kernel<8> : stream_digits_kernel<4>, digit_ctas(per_token) * m, kRowThreads,
+                stream, x, x_type, digits, e, columns, column_tiles(per_token * m), vector);
 }
 
 bool stream_scaled_serves(const StreamScaledArgs& a) {
