@@ -117,9 +117,9 @@ __device__ __forceinline__ uint4 load_activations(const uint8_t* src) {
 // Only where the matrix is not much more than the CTAs of one round ask for at once: from there on the requests stand in the
 // way of the loads (us, with it | without: int8 16 rows 2048 x 2048 4.6 | 5.1, 4096 x 4096 7.6 | 8.0; 8192 x 4096
 // 10.5 | 10.2, 14336 x 8192 36 | 31, one token 28672 x 8192 68 | 54; uint4 16 tokens 8192 x 4096 13.5 | 12.8,
-// 14336 x 4096 24.2 | 23.2, 28672 x 8192 88 | 78; f32 tokens 4096 x 4096 14.1 | 14.9; groups of 32, 16 tokens 11008 x 4096
-// 37 | 45, 14336 x 8192 89 | 87). `steps_of_64`: of a scaled product, whose loads are the larger ones.
-constexpr long long prefetch_limit(bool steps_of_64) { return steps_of_64 ? 1LL << 24 : (1LL << 25) - 1; }
+// 14336 x 4096 24.2 | 23.2, 28672 x 8192 88 | 78; f32 tokens 4096 x 4096 14.1 | 14.9). `rows` 0: nothing (an empty range
+// and not a branch around the loop, behind which the loads of 16 tokens with groups of 32 on 11008 x 4096 took 45 us, not 38).
+constexpr long long kIntPrefetchBytes = (1LL << 25) - 1, kScaledPrefetchBytes = 1LL << 24;
 __device__ __forceinline__ void prefetch_rows(const uint8_t* codes, long long row_bytes, long long row0, int rows,
                                               long long total_rows) {
   const long long last = row0 + rows < total_rows ? row0 + rows : total_rows;
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(kThreads, CTAS) stream_int_kernel(const IntPar
   const int g = lane >> 2, t = lane & 3;
   const int row0 = blockIdx.x * kR;
   launch_dependents();
-  if (p.prefetch != 0) prefetch_rows(p.codes, p.row_bytes, row0, kR, p.rows);
+  prefetch_rows(p.codes, p.row_bytes, row0, p.prefetch != 0 ? kR : 0, p.rows);
 
   // (offsets from the CTA's first row: a pointer per row would be two registers)
   const uint8_t* codes = p.codes + row0 * p.row_bytes + t * (kNibbles ? 8 : 16);
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(kThreads, CTAS) stream_scaled_kernel(const Sca
   const int g = lane >> 2, t = lane & 3;
   const int row0 = blockIdx.x * kR;
   launch_dependents();
-  if (p.prefetch != 0) prefetch_rows(p.codes, p.row_bytes, row0, kR, p.rows);
+  prefetch_rows(p.codes, p.row_bytes, row0, p.prefetch != 0 ? kR : 0, p.rows);
 
   // (offsets from the CTA's first row: a pointer per row would be two registers)
   const uint8_t* codes = p.codes + row0 * p.row_bytes + t * kBytes;
@@ -1042,7 +1042,7 @@ qx_status launch_stream_int(const StreamIntArgs& a, cudaStream_t stream) {
   p.activation = a.activation;
   p.y_type = a.y_type;
   p.prepared = a.prepared ? 1 : 0;
-  p.prefetch = p.row_bytes * a.rows <= prefetch_limit(false) ? 1 : 0;
+  p.prefetch = p.row_bytes * a.rows <= kIntPrefetchBytes ? 1 : 0;
   p.digits = a.digits;
   switch (a.source) {
     case kStreamBytes:
@@ -1111,7 +1111,7 @@ qx_status launch_stream_scaled(const StreamScaledArgs& a, void* scratch, cudaStr
   p.activation = a.activation;
   p.y_type = a.y_type;
   p.flush_steps = promote_columns(a) / step;
-  p.prefetch = p.row_bytes * a.rows <= prefetch_limit(step == 64) ? 1 : 0;
+  p.prefetch = p.row_bytes * a.rows <= kScaledPrefetchBytes ? 1 : 0;
   const bool bf16 = a.x_type != QX_STORAGE_F16;
   return a.source == kStreamBytes ? launch_scaled<kStreamBytes>(p, bf16, planes, step, fragments, stream)
                                   : launch_scaled<kStreamNibbles>(p, bf16, planes, step, fragments, stream);
