@@ -34,9 +34,11 @@ namespace {
 //     8192 x 28672 52 | 49
 //   24 rows: 4096 x 4096 8.8 | 10.4;  2048 x 8192 13.4 | 14.5;  4096 x 11008 18.5 | 18.9;  4096 x 28672 41.9 | 40.6;
 //     5120 x 5120 15.2 | 11.7
-//   32 rows, a whole tile of tokens there: 1024 x 1408 4.6 | 4.1;  4096 x 4096 9.2 | 8.1
+//   32 rows, a whole tile of tokens there: 1024 x 1024 3.5 | 3.8;  2000 x 2048 5.4 | 5.5;  1000 x 4096 7.2 | 7.5;
+//     3000 x 4096 8.5 | 7.9
 bool few_rows(const Int8GemmArgs& a) {
-  if (a.n <= 4096 && a.m <= kStreamW8A8Rows) return a.m <= 16 || a.k <= 16384;
+  if (a.m == kStreamW8A8Rows) return a.n <= 4096 && a.n * a.k <= (1LL << 22);
+  if (a.n <= 4096 && a.m < kStreamW8A8Rows) return a.m <= 16 || a.k <= 16384;
   return a.n <= 8192 && a.m <= 16 && a.k <= 16384;
 }
 bool stream_route(const Int8GemmArgs& a, StreamIntArgs* s) {

@@ -14,7 +14,7 @@ enum StreamSource {
 
 constexpr int kStreamColumns = 64;  // activation rows (digit planes: four or eight per token) at most
 
-constexpr int kStreamW8A8Rows = 31;  // of W8A8
+constexpr int kStreamW8A8Rows = 32;  // of W8A8
 
 // ---- whole numbers on both sides (one weight scale per row) --------------------------------
 // What becomes of a row's exact int32 sums.
