@@ -114,12 +114,16 @@ __device__ __forceinline__ uint4 load_activations(const uint8_t* src) {
 
 // Calls a CTA's rows of codes into L2. Before the wait for the kernel in front this reads nothing
 // on the program's behalf: should that kernel write these bytes, the lines in L2 change with them.
-// Only where the matrix is not much more than the CTAs of one round ask for at once: from there on the requests stand in the
-// way of the loads (us, with it | without: int8 16 rows 2048 x 2048 4.6 | 5.1, 4096 x 4096 7.6 | 8.0; 8192 x 4096
-// 10.5 | 10.2, 14336 x 8192 36 | 31, one token 28672 x 8192 68 | 54; uint4 16 tokens 8192 x 4096 13.5 | 12.8,
-// 14336 x 4096 24.2 | 23.2, 28672 x 8192 88 | 78; f32 tokens 4096 x 4096 14.1 | 14.9). `rows` 0: nothing (an empty range
-// and not a branch around the loop, behind which the loads of 16 tokens with groups of 32 on 11008 x 4096 took 45 us, not 38).
-constexpr long long kIntPrefetchBytes = (1LL << 25) - 1, kScaledPrefetchBytes = 1LL << 24;
+// Matrices of up to 32 MB as a whole. Of larger ones the requests of all CTAs stand in the way of the loads: the first 24 MB
+// of whole numbers, whose first CTAs wait for the kernel in front anyway, and nothing with scales along K. Measured (us, none |
+// 24 MB | all; graph replay, codes from memory): int8 one token 4096 x 4096 7.3 | 6.9 | 6.9, 14336 x 4096 16.8 | 16.1 | 17.5,
+// 28672 x 8192 54 | 52 | 67, 8192 x 16384 33.5 | 30.8 | 35.1, W8A8 1024 x 28672 34.3 | 36.5 | 35.4;  uint4 five tokens
+// 4096 x 14336 18.8 | 20.7 | 19.9, 16 tokens 14336 x 4096 23.2 | 23.3 | 23.5, 28672 x 8192 78 | 79 | 88. Three matrices in
+// turn, partly in L2: W8A8 1024 x 28672 33.1 | 34.5 | 28.0, int8 14336 x 4096 17.1 | 16.2 | 15.5, uint4 five tokens 18.5 |
+// 18.4 | 17.4.
+// (`rows` 0: an empty range and not a branch around the loop, behind which the loads of 16 uint4 tokens with groups of 32 on
+// 11008 x 4096 took 45 us, not 38.)
+constexpr long long kPrefetchWhole = 1LL << 25, kPrefetchFirst = 24LL << 20;
 __device__ __forceinline__ void prefetch_rows(const uint8_t* codes, long long row_bytes, long long row0, int rows,
                                               long long total_rows) {
   const long long last = row0 + rows < total_rows ? row0 + rows : total_rows;
@@ -155,7 +159,7 @@ struct IntParams {
   int32_t* acc;
   long long row_bytes, x_stride, ldy;
   int rows, columns, x_rows, steps;
-  int prefetch, activation, y_type, prepared, digits;
+  int prefetch_rows, activation, y_type, prepared, digits;
 };
 
 // A step is 64 columns: 16 per lane of a quad (16 bytes of int8, 8 bytes of nibbles).
@@ -172,7 +176,7 @@ __global__ void __launch_bounds__(kThreads, CTAS) stream_int_kernel(const IntPar
   const int g = lane >> 2, t = lane & 3;
   const int row0 = blockIdx.x * kR;
   launch_dependents();
-  prefetch_rows(p.codes, p.row_bytes, row0, p.prefetch != 0 ? kR : 0, p.rows);
+  prefetch_rows(p.codes, p.row_bytes, row0, row0 < p.prefetch_rows ? kR : 0, p.rows);
 
   // (offsets from the CTA's first row: a pointer per row would be two registers)
   const uint8_t* codes = p.codes + row0 * p.row_bytes + t * (kNibbles ? 8 : 16);
@@ -375,7 +379,7 @@ struct ScaledParams {
   long long row_bytes, x_stride, ldy;
   uint32_t nibble_xor;
   int rows, columns, m, steps, group, groups, flush_steps;
-  int prefetch, activation, y_type;
+  int prefetch_rows, activation, y_type;
 };
 
 // A step is 64 columns, or 32 where sums of 32 leave the tensor core: a quarter per lane of a quad.
@@ -396,7 +400,7 @@ __global__ void __launch_bounds__(kThreads, CTAS) stream_scaled_kernel(const Sca
   const int g = lane >> 2, t = lane & 3;
   const int row0 = blockIdx.x * kR;
   launch_dependents();
-  prefetch_rows(p.codes, p.row_bytes, row0, p.prefetch != 0 ? kR : 0, p.rows);
+  prefetch_rows(p.codes, p.row_bytes, row0, row0 < p.prefetch_rows ? kR : 0, p.rows);
 
   // (offsets from the CTA's first row: a pointer per row would be two registers)
   const uint8_t* codes = p.codes + row0 * p.row_bytes + t * kBytes;
@@ -930,6 +934,10 @@ constexpr long long kWideRows = 2 * 148 * 16 + 1;
 // one token 5120 x 5120 10.5 | 9.0, W4A8 16 rows 11.7 | 10.8.
 constexpr long long kWideRowsOfFew = 32 * 192;
 
+int prefetched_rows(long long row_bytes, long long rows, long long of_more) {
+  return static_cast<int>(row_bytes * rows <= kPrefetchWhole ? rows : of_more / row_bytes);
+}
+
 int column_tiles(long long columns) { return columns <= 8 ? 1 : (columns <= 16 ? 2 : (columns <= 32 ? 4 : 8)); }
 
 template <StreamSource SRC, bool FRAGMENTS, int NT>
@@ -1042,7 +1050,7 @@ qx_status launch_stream_int(const StreamIntArgs& a, cudaStream_t stream) {
   p.activation = a.activation;
   p.y_type = a.y_type;
   p.prepared = a.prepared ? 1 : 0;
-  p.prefetch = p.row_bytes * a.rows <= kIntPrefetchBytes ? 1 : 0;
+  p.prefetch_rows = prefetched_rows(p.row_bytes, a.rows, kPrefetchFirst);
   p.digits = a.digits;
   switch (a.source) {
     case kStreamBytes:
@@ -1111,7 +1119,7 @@ qx_status launch_stream_scaled(const StreamScaledArgs& a, void* scratch, cudaStr
   p.activation = a.activation;
   p.y_type = a.y_type;
   p.flush_steps = promote_columns(a) / step;
-  p.prefetch = p.row_bytes * a.rows <= kScaledPrefetchBytes ? 1 : 0;
+  p.prefetch_rows = prefetched_rows(p.row_bytes, a.rows, 0);
   const bool bf16 = a.x_type != QX_STORAGE_F16;
   return a.source == kStreamBytes ? launch_scaled<kStreamBytes>(p, bf16, planes, step, fragments, stream)
                                   : launch_scaled<kStreamNibbles>(p, bf16, planes, step, fragments, stream);
