@@ -1046,19 +1046,22 @@ def _extra_canonical(qx, wl, torch, hbm_peak):
         xd = torch.from_numpy(rng.standard_normal((m, k), dtype=np.float32)).cuda().to(torch.bfloat16)
         bias = torch.from_numpy(rng.standard_normal(n, dtype=np.float32)).cuda()
         yd = torch.zeros((m, n), dtype=torch.bfloat16, device="cuda")
-        sec = _time_calls(torch, lambda i: qx.check(
-            handles[i % copies].qgemm_storage_dev(xd, qx.BF16, yd, qx.BF16, m, bias=bias,
-                                                  activation=qx.ACT_SILU), "canonical"),
-            4 * copies if m < 32 else 4)
+        def call(i):
+            qx.check(handles[i % copies].qgemm_storage_dev(xd, qx.BF16, yd, qx.BF16, m, bias=bias,
+                                                           activation=qx.ACT_SILU), "canonical")
+        sec = _time_calls(torch, call, 4 * copies if m < 32 else 4)
+        launches = qx.launch_count()
+        call(0)
+        launches = qx.launch_count() - launches
         nbytes = (code_bytes + 4 * n * groups * (2 if layout == qx.UINT4_AFFINE else 1) + 2 * m * k +
                   4 * n + 2 * m * n)
         name = {qx.INT8_SYMMETRIC: "int8", qx.INT4_SYMMETRIC: "int4g128",
                 qx.UINT4_AFFINE: "uint4affine_g128"}[layout] + f"_m{m}_n{n}_k{k}"
         out[name] = {"us": sec * 1e6, "gbs": nbytes / sec / 1e9,
                      "frac_of_measured_hbm": nbytes / sec / 1e9 / hbm_peak,
-                     # the digits of the activations, then the projection; from five tokens on
-                     # row digits, the W8A8 tensor-core GEMM on the digit planes and the combine per 256 tokens
-                     "launches": 2 if (m < 5 or layout != qx.INT8_SYMMETRIC) else 3 * ((m + 255) // 256)}
+                     # (where a call has more than one: the activations' digits or order in front of the projection; for
+                     # long int8 batches digit planes, the W8A8 tensor-core GEMM and their sum per 256 tokens)
+                     "launches": launches}
         if m >= 32:
             out[name]["tops"] = 2.0 * m * n * k / sec / 1e12
         for h in handles:

@@ -25,26 +25,26 @@
 //           multiply-adds on exactly converted codes, every weight decoded on its own as in
 //           the reference (scale * code, or scale * (nibble - zero)).
 // With an act-order map the activations are first gathered into packed column order.
-//   streamed small batches (qx_stream_mma.cu, chosen by stream_digits_route and stream_scaled_route below): up to 16 tokens of
-//           int8 tensors with one scale per row, five to 32 of the others;
-//   tensor cores (int8 with one scale per row, five tokens or more): four digit planes under a
-//           per-token envelope through the W8A8 GEMM; see "long prefills" below.
+//   streamed small batches (qx_stream_mma.cu, chosen by stream_digits_route and stream_scaled_route below): one to four
+//           tokens of int8 tensors with one scale per row (digits under one envelope per token, and those of the
+//           remainders), up to 16 on few rows; five to 32 of the others;
+//   tensor cores (larger batches of int8 with one scale per row, from five tokens on): four digit planes under a
+//           per-token envelope through the W8A8 GEMM; see "tensor cores" below.
 //   tensor cores with scales applied per group (batches of the 4-bit and group-scaled tensors):
 //           qx_scaled_gemm.cu, chosen by scaled_route below.
 // Inputs stored as f16 / bf16 are widened exactly, the output is rounded once at the store.
-// On the first two paths a token's result does not depend on the batch it is computed in; a
-// batch that crosses a line of a tensor-core route changes route and with it the rounding (same
-// tolerance).
+// On the first two paths a token's result does not depend on the batch it is computed in, nor on one to four streamed
+// tokens; a batch that crosses a line of another route changes route and with it the rounding (same tolerance).
 //
 // HBM layout. Codes stay in the canonical row-major byte order (a row of K int8 codes or
 // K/2 nibble pairs is already what a warp wants to stream with 16-byte loads), followed by
 // the f32 scale table [rows][groups]. Nothing is re-tiled, so prepared bytes = canonical
-// bytes. The digit images of a call's activations (1792 bytes per token and 512 columns)
-// live in the device's default workspace.
+// bytes. The digit images of a call's activations (1792 bytes per token and 512 columns) and what the other routes put
+// in front of their products live in the call's workspace.
 //
 // Kernels. CUDA cores and warp-level MMAs for decode-sized batches, the tcgen05 W8A8 GEMM for int8 prefills.
-// Measured on 14336 x 4096 int8 with one bf16 token: 15.6 us per call for both launches (digits and the projection behind
-// them), 17.2 on the dp4a digit kernels, 24 on the float path.
+// Measured on 14336 x 4096 int8 with one bf16 token, graph replay: 16.1 us per call for both launches (digits and the
+// projection behind them), 17.3 on the dp4a digit kernels, 24 on the float path.
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -840,10 +840,9 @@ __global__ void __launch_bounds__(256) gather_activations_kernel(const void* __r
   }
 }
 
-// ---- five tokens or more of int8 tensors with one scale per row: the tensor cores ----------
-// (Measured on 14336 x 4096 / 4096 x 4096: 4 tokens 23.7 / 18.1 us here against 34.4 / 14.8 us
-// on the digit kernel, 8 tokens 21.7 / 16.3 against 56.5 / 19.5, 16 tokens 22.8 / 16.8 against
-// 102.8 / 33.9.) Four digit planes of the activations become four int8 "token" rows each
+// ---- batches of int8 tensors with one scale per row: the tensor cores ----------------------
+// (From five tokens on, where stream_digits_route below does not take them. Measured on 14336 x 4096: 5 tokens 19.0 us, 8
+// 16.9, 16 17.2; the digit kernel 56.5 and 102.8 for 8 and 16.) Four digit planes of the activations become four int8 "token" rows each
 // and the W8A8 tensor-core GEMM (qx_int8_gemm_tc.cu) forms the exact integer sums
 //   A_d[t, o] = sum_k code[o, k] * p_d[t, k],      d = 0 .. 3,
 // over the whole row. The envelope is therefore one power of two per TOKEN, not per 16
@@ -853,8 +852,8 @@ __global__ void __launch_bounds__(256) gather_activations_kernel(const void* __r
 // four it is below the f32 roundings that follow. The GEMM's own epilogue scales float(A_d) by
 // the weight scale of the channel and by e * 256^d (two rounded multiplies), and a last kernel
 // adds the four planes, the bias, applies the activation and stores the output type.
-// |A_d| <= K * 128 * 128 fits int32 for K <= 131000 (the GEMM's own limit). Tokens whose
-// largest magnitude is below 2^-70 count as zero.
+// |A_d| <= K * 128 * 128 fits int32 for K <= 131000 (the GEMM's own limit). The envelope is 2^-69 at least: an
+// activation below 2^-100 counts as zero.
 constexpr long long kPrefillTokens = 5;
 constexpr long long kPrefillChunk = 256;  // tokens per GEMM launch: bounds the scratch
 constexpr int kPlanes = 4;
@@ -1045,15 +1044,15 @@ bool scaled_route(const qx_canonical_weights* w, int x_type, long long m) {
 // other route (us):
 //   int8, one scale per row (exact sums, eight digit rows per token up to four tokens, then four; other route: digit kernel
 //   up to four tokens, then digit planes through the W8A8 GEMM):
-//     1 token: 1024 x 1024 3.6 | 3.7, 4096 x 4096 7.2 | 9.3, 14336 x 4096 16.8 | 17.3, 28672 x 8192 54 | 55;
-//     4: 4096 x 4096 9.5 | 16.9, 14336 x 4096 22.9 | 34.5, 28672 x 8192 68 | 115
+//     1 token: 1024 x 1024 3.4 | 3.7, 4096 x 4096 7.0 | 9.3, 14336 x 4096 16.1 | 17.3, 28672 x 8192 52 | 55;
+//     4: 4096 x 4096 9.5 | 16.9, 14336 x 4096 22.5 | 34.5, 28672 x 8192 68 | 115
 //     5: 5120 x 5120 13.1 | 16.1, 8192 x 4096 12.0 | 15.5, 14336 x 4096 21.2 | 19.0;  8: 4096 x 11008 20.1 | 22.3,
 //     8192 x 4096 12.8 | 13.8, 11008 x 4096 20.5 | 15.8, 28672 x 8192 66 | 50
 //     9: 4096 x 4096 11.7 | 13.9, 6144 x 4096 20.5 | 14.8;  15: 4096 x 8192 20.7 | 20.8;  16: 4096 x 4096 13.1 | 13.0,
 //     2048 x 8192 18.8 | 17.4, 4096 x 11008 25.0 | 22.8
 //   16-bit tokens, scales along K (uint4, groups of 128; other route: qx_scaled_gemm.cu): 14336 x 4096: 8 tokens 18.7 | 31.2,
 //     16: 23.2 | 32.2, 17: 36.8 | 32.6;  4096 x 4096: 32: 10.8 | 19.9;  5120 x 5120: 17: 23.6 | 22.7;  8192 x 4096: 32:
-//     20.3 | 24.3;  28672 x 8192: 16: 78 | 93;  4096 x 14336: 32: 31.7 | 34.8;  groups of 32: 11008 x 4096, 16: 37 | 45
+//     20.3 | 24.3;  28672 x 8192: 16: 78 | 93;  4096 x 14336: 32: 31.7 | 34.8;  groups of 32: 11008 x 4096, 16: 38 | 45
 //   f32 tokens (three planes; other route: the digit kernels up to 24 tokens): 14336 x 4096: 16: 42 | 121;  4096 x 4096:
 //     24: 21.4 | 59, 32: 22.1 | 25.9;  5120 x 5120: 24: 42 | 85, 32: 42 | 29;  1024 x 2048: 17: 11.3 | 10.5, 32: 11.5 | 18.5
 // Not the smallest products, which are launches and nothing else on either route; and up to four tokens with scales
@@ -1161,7 +1160,7 @@ qx_status launch_canonical(const qx_canonical_weights* w, const void* x, int x_t
   // workspace behind its counters: [gathered activations (act-order)][digit images]
   const size_t gather_bytes =
       w->act_order != nullptr ? align_up(static_cast<size_t>(m) * w->columns * sizeof(float), 256) : 0;
-  // int8 with one scale per row, five tokens or more: the tensor-core route
+  // int8 with one scale per row, from here on: the tensor-core route, where nothing streams
   long long prefill_from = kPrefillTokens;
   // developer switches: QX_B200_CANONICAL_PREFILL_TOKENS=<n> moves the threshold, and from there on nothing streams; nor
   // where the digit planes are to take the CUDA-core GEMM

@@ -15,7 +15,7 @@
 //
 // Pipeline (persistent CTAs, one per SM, 320 threads):
 //   warp 0      TMA producer: 128-byte-swizzled K-slabs of W (128 x 128 B) and X
-//               (BN x 128 B) into a 4-stage shared-memory ring (full/empty mbarriers)
+//               (BN x 128 B) into a shared-memory ring of three to eight stages (full/empty mbarriers)
 //   warp 1      MMA issuer: one thread issues tcgen05.mma kind::i8 (K = 32 per
 //               instruction, four per slab) into one of two TMEM accumulators
 //   warps 2-9   epilogue: tcgen05.ld -> int->f32 -> scale -> global stores, overlapped

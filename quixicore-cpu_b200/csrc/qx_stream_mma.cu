@@ -8,16 +8,16 @@
 // the fixed costs around that. A pipeline of specialised warps over 128-row tiles (qx_scaled_gemm.cu,
 // qx_int8_gemm_tc.cu) has few CTAs here and 8 us of start and end. So: no shared memory and no
 // barriers on the way of the weights. A warp owns 16 or 32 weight rows and one contiguous part of
-// K (eight warps of a CTA share the rows); its lanes load codes straight into registers, several
-// steps ahead, in the places where the warp-level MMA wants them as its A operand: lane (g, t)
+// K (eight warps of a CTA share the rows); its lanes load codes straight into registers, two
+// or four steps ahead, in the places where the warp-level MMA wants them as its A operand: lane (g, t)
 // holds rows g and g + 8 and a quarter of a step's columns, in one piece. Which columns an MMA slot
 // stands for is free as long as both operands agree: the B operand is read through L1 with 16-byte loads,
 // from the activations' rows as they are (W8A8, up to eight 16-bit tokens), or where a kernel in front
 // writes them anyway, or for more tokens, from the order in which the lanes read them (plain rows cost a
 // load eight lines). The parts of K meet in shared memory at the end, in exact integers or in 64 bits.
 //
-// Measured (us, before | here): W4A8 16 rows 4096 x 4096 22.6 | 8.3; W8A8 4 rows 1024 x 1408 6.2 | 2.9; int8 1 token
-// 14336 x 4096 17.2 | 15.6 (3.8 TB/s); uint4 16 tokens 14336 x 4096 31.8 | 22.8 (1.4 TB/s). 16-bit activations are bound
+// Measured (us, before | here, codes from memory): W4A8 16 rows 4096 x 4096 22.6 | 8.2; W8A8 4 rows 1024 x 1408 6.0 | 3.0; int8
+// 1 token 14336 x 4096 17.3 | 16.1 (3.7 TB/s); uint4 16 tokens 14336 x 4096 32.2 | 23.5. 16-bit activations are bound
 // by the latency of loads at four warps per scheduler (more than half of the cycles between two instructions of a
 // warp), which the registers of 32 rows x 16 tokens leave no room to ask for earlier.
 //
